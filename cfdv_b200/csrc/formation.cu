@@ -1,6 +1,6 @@
 // CUDA kernels for the per-step FDV set-up: element formation (+ ApplyBC) and the
 // CFL time step.  Formation is one thread block per element running the phases of
-// formation.cuh; the CFL step is a per-element minimum with a deterministic
+// formation.cuh (quad4) or formation_hex.cuh (hex8); the CFL step is a per-element minimum with a deterministic
 // two-level reduction.
 #include <cuda_runtime.h>
 
@@ -9,30 +9,66 @@
 
 namespace cfdv {
 
-template <int NDIM>
-__global__ void __launch_bounds__(FormTraits<NDIM>::THREADS, FormTraits<NDIM>::MIN_BLOCKS)
-    fdv_form_kernel(FormArgs a) {
-  __shared__ FormShared<NDIM> sh;
-  __shared__ int bad;
-  const int tid = threadIdx.x;
-  if (tid == 0) bad = 0;
-  for (int e = blockIdx.x; e < a.n_elements; e += gridDim.x) {
-    form_step<NDIM>(0, a, sh, e, tid, &bad);
+// one 64-thread block per quad4 element (formation.cuh)
+__global__ void __launch_bounds__(FormTraits<2>::THREADS, FormTraits<2>::MIN_BLOCKS) fdv_form_quad_kernel(FormArgs a) {
+  __shared__ FormShared<2> sh;
+  const int tid = threadIdx.x, e = blockIdx.x;
+  int bad = 0;
+  form_step<2>(0, a, sh, e, tid, &bad);
+  __syncthreads();
+  const int n = form_nsteps<2>(sh);
+  for (int k = 1; k < n; k++) {
+    form_step<2>(k, a, sh, e, tid, &bad);
     __syncthreads();
-    const int n = form_nsteps<NDIM>(sh);
-    for (int k = 1; k < n; k++) {
-      form_step<NDIM>(k, a, sh, e, tid, &bad);
-      __syncthreads();
-    }
   }
-  if (tid == 0 && bad) atomicOr(a.status, STATUS_NONFINITE_MATRIX);
+  if (bad) atomicOr(a.status, STATUS_NONFINITE_MATRIX);
+}
+
+// one 128-thread block per hex8 element (formation_hex.cuh)
+__global__ void __launch_bounds__(FormTraits<3>::THREADS, CFDV_FORM3D_BLOCKS) fdv_form_hex_kernel(FormArgs a) {
+  __shared__ FormShared<3> sh;
+  const int tid = threadIdx.x, e = blockIdx.x;
+  int bad = 0;
+  hex_load(a, sh, e, tid);
+  __syncthreads();
+  hex_geom_jac(sh, tid);
+  __syncthreads();
+  hex_dphi(a, sh, tid);
+  __syncthreads();
+  hex_state<false>(sh, 0, tid);
+  __syncthreads();
+  hex_gp_domain(a, sh, tid);
+  __syncthreads();
+  hex_rows<false>(a, sh, tid);
+  __syncthreads();
+  hex_hmat<false>(a, sh, tid);
+  __syncthreads();
+  hex_contract<false>(sh, tid);
+  __syncthreads();
+  const int nf = sh.nfaces;
+  for (int lf = 0; lf < nf; lf++) {
+    hex_face_geom(a, sh, lf, tid);
+    __syncthreads();
+    hex_state<true>(sh, lf, tid);
+    __syncthreads();
+    hex_gp_face(a, sh, lf, tid);
+    __syncthreads();
+    hex_rows<true>(a, sh, tid);
+    __syncthreads();
+    hex_hmat<true>(a, sh, tid);
+    __syncthreads();
+    hex_contract<true>(sh, tid);
+    __syncthreads();
+  }
+  hex_write(a, sh, e, tid, &bad);
+  if (bad) atomicOr(a.status, STATUS_NONFINITE_MATRIX);
 }
 
 cudaError_t launch_form(int ndim, const FormArgs& a, cudaStream_t st) {
   if (a.n_elements <= 0) return cudaSuccess;
   const int grid = a.n_elements;
-  if (ndim == 2) fdv_form_kernel<2><<<grid, FormTraits<2>::THREADS, 0, st>>>(a);
-  else fdv_form_kernel<3><<<grid, FormTraits<3>::THREADS, 0, st>>>(a);
+  if (ndim == 2) fdv_form_quad_kernel<<<grid, FormTraits<2>::THREADS, 0, st>>>(a);
+  else fdv_form_hex_kernel<<<grid, FormTraits<3>::THREADS, 0, st>>>(a);
   return cudaGetLastError();
 }
 

@@ -1,4 +1,6 @@
-// FDV element formation as the phases of one thread block ("CTA") per element.
+// FDV element formation as the phases of one thread block ("CTA") per element: the pieces shared
+// by both dimensions and by the adjoint, and the steps of a quad4 element (2D).  The steps of a
+// hex8 element (3D) are in formation_hex.cuh.
 //
 // Per element the CTA computes what the reference builds in FDVGalerkin::operator()
 // (FDV/FDVGalerkin.h:121-154) followed by ApplyBC (FDV/Function/ApplyBC.h:14-133):
@@ -14,7 +16,7 @@
 //             (FDVGalerkin.h:405-451)
 //   faces     same three phases per boundary face with 0 != bc < 100
 //             (FDVGalerkin.h:455-533, 643-756; TFNorm2D TestFunctions1D.h:73-82,
-//             TFNorm3D calc_TF_norm3D.h:9-167, eval1dboundary.h, eval2dboundary.h)
+//             eval1dboundary.h)
 //   write     ApplyBC through the precomputed Dirichlet row mask, then a coalesced
 //             store of R (column-major, FP64 or FP32) and rhs.
 // Every phase is a host/device function of (block state, thread id) so that the
@@ -43,9 +45,9 @@ struct FormTraits {
   // p = (r*NEQ + s)*NNOD + N, with one accumulator per column node M
   static constexpr int NPAIR = NNOD * RS;
   static constexpr int PAIRS = (NPAIR + THREADS - 1) / THREADS;
-  // coefficient rows per Gauss point for the column node M: Phi_M, dPhi_M,j (j < NDIM) and,
-  // in 2D, S_M = sum_j dPhi_M,j for the upwind term
-  static constexpr int NCOEF = 1 + NDIM + (NDIM == 2 ? 1 : 0);
+  // coefficient rows per Gauss point for the column node M: Phi_M, dPhi_M,j (j < NDIM) and
+  // S_M = sum_j dPhi_M,j for the upwind term
+  static constexpr int NCOEF = 2 + NDIM;
   static constexpr int MIN_BLOCKS = (NDIM == 2) ? 12 : CFDV_FORM3D_BLOCKS;  // resident blocks per SM (register cap)
 };
 
@@ -125,10 +127,10 @@ CFDV_HD CFDV_INLINE void hnm_face_phi_3d(const double* H, int f, double* phib) {
 template <int NDIM>
 struct GpGeom {  // isoparametric map at the Gauss point (dead once the flow state exists)
   double jac[3][3];  // dx_i / dxi_k
-  double inv[3][3];  // adjugate (3D)
+  double inv[3][3];  // unused in 2D
   double iJ;         // 1 / det
   double dPxi[FormTraits<NDIM>::NNOD][3];
-  double pjac[NDIM == 2 ? 3 : 1][3];  // 2D adaptive element: Jacobian of the plain shape functions
+  double pjac[3][3];  // adaptive element: Jacobian of the plain shape functions
 };
 
 template <int NDIM>
@@ -166,6 +168,7 @@ struct FormShared {
   double dt, dtsq_2;                  // time step of the formation and dt^2 / 2
   double rhs[T::KE];
   GpSlot<NDIM> slot[T::Q];
+  static_assert(NDIM == 2, "the hex8 element has its own steps");
   union {
     // A(q, i) = a + b and D(q, i) = s2 a + s4 b of the domain Gauss points (a, b until step 7)
     double AD[T::Q][2][NDIM][25];
@@ -296,10 +299,10 @@ CFDV_HD CFDV_INLINE void step_geom_jac(const FormArgs& a, FormShared<NDIM>& sh, 
     const int q = tid / (NDIM * NDIM), i = (tid / NDIM) % NDIM, k = tid % NDIM;
     GpSlot<NDIM>& sl = sh.slot[q];
     sl.g.jac[i][k] = geom_jac_entry<T::NNOD>(sl.g.dPxi, sh.nd, i, k);
-    if (NDIM == 2 && sh.hnm >= 0 && i == 0 && k == 0) {
+    if (sh.hnm >= 0 && i == 0 && k == 0) {
       double z[3];
       gp_point<NDIM>(a, q, z);
-      const double* x4[4] = {sh.nd[0].x, sh.nd[1].x, sh.nd[2].x, sh.nd[3 % T::NNOD].x};
+      const double* x4[4] = {sh.nd[0].x, sh.nd[1].x, sh.nd[2].x, sh.nd[3].x};
       plain_jac_2d(z, x4, sl.g.pjac);
     }
   }
@@ -336,7 +339,7 @@ CFDV_HD CFDV_INLINE void step_dphi(FormShared<NDIM>& sh, int tid) {
       sl.cM[1 + j][N] = sl.dPhi[N][j];
       sd += sl.dPhi[N][j];
     }
-    if (NDIM == 2) sl.cM[T::NCOEF - 1][N] = sd;
+    sl.cM[T::NCOEF - 1][N] = sd;
   }
 }
 
@@ -461,8 +464,7 @@ CFDV_HD CFDV_INLINE void step_stress(const FormArgs& a, FormShared<NDIM>& sh, in
     sl.st.mu = gas_mu(a.gas, sl.st.T);
     sl.st.k = gas_k(a.gas, sl.st.mu);
     viscous_stress<NDIM>(sl.st);
-    for (int N = 0; N < T::NNOD; N++) sl.Psi[N] = 0.0;  // 3D: tau = 0, no upwinding
-    if constexpr (NDIM == 2) supg_psi_2d(sh, sl);
+    supg_psi_2d(sh, sl);
   }
 }
 
@@ -473,11 +475,10 @@ CFDV_HD CFDV_INLINE void flux_sums(const FormArgs& a, const FormShared<NDIM>& sh
   constexpr int NN = Pass<NDIM, FACE>::NN;
   double Fbar[NDIM], divF = 0.0;
   for (int i = 0; i < NDIM; i++) Fbar[i] = 0.0;
-  const bool withF = (NDIM == 2) || a.physical_3d_flux;
   for (int b = 0; b < NN; b++) {
     const NodePrim& nb = pass_node<NDIM, FACE>(sh, fc, b);
     for (int i = 0; i < NDIM; i++) {
-      const double fg = node_flux_entry<NDIM>(sl.st, nb, a.gas.creyn, withF, i, r);
+      const double fg = node_flux_entry<NDIM>(sl.st, nb, a.gas.creyn, true, i, r);
       Fbar[i] += sl.Phi[b] * fg;
       divF += sl.dPhi[b][i] * fg;
     }
@@ -495,11 +496,9 @@ CFDV_HD CFDV_INLINE void step_jacobians(const FormArgs& a, FormShared<NDIM>& sh,
   constexpr int Q = Pass<NDIM, FACE>::NQ, NEQ = T::NEQ;
   constexpr int C0 = 0, CN = Q * NDIM;                     // c: (q, i)
   constexpr int B0 = 32, BN = Q * NDIM;                    // b: (q, i)
-  constexpr int A0 = (NDIM == 3) ? 104 : 8;                // a: q
-  constexpr int F0 = (NDIM == 3) ? 64 : 40, FN = Q * NEQ;  // flux sums: (q, r)
-  static_assert(CN <= B0 && B0 + BN <= F0 && F0 + FN <= T::THREADS && A0 + Q <= T::THREADS &&
-                    (NDIM == 2 ? (CN <= A0 && A0 + Q <= B0) : (F0 + FN <= A0)),
-                "task ranges overlap");
+  constexpr int A0 = 8;                                    // a: q
+  constexpr int F0 = 40, FN = Q * NEQ;                     // flux sums: (q, r)
+  static_assert(CN <= A0 && A0 + Q <= B0 && B0 + BN <= F0 && F0 + FN <= T::THREADS, "task ranges overlap");
   if (tid >= C0 && tid < C0 + CN) {
     GpSlot<NDIM>& sl = sh.slot[(tid - C0) / NDIM];
     const int i = (tid - C0) % NDIM;
@@ -576,7 +575,7 @@ CFDV_HD CFDV_INLINE void step_hmat_rhs(const FormArgs& a, FormShared<NDIM>& sh, 
   }
 }
 // Domain contraction, factored through the row node N:
-//   R(N r, M s) = sum_q [ Phi_M G0 + sum_j dPhi_M,j G1j (+ S_M G2 in 2D) ]  with
+//   R(N r, M s) = sum_q [ Phi_M G0 + sum_j dPhi_M,j G1j + S_M G2 ]  with
 //   G0  = wJ (Phi_N delta_rs - sum_i dPhi_N,i X_i(r,s)),
 //   G1j = wJ sum_i dPhi_N,i h_ij(r,s),   G2 = wJ Psi_N sum_i X_i(r,s),
 // which is sum_k B_k(N,M) C_k(r,s) of FDVGalerkin.h:405-451 regrouped (S_M = sum_j dPhi_M,j).
@@ -603,11 +602,9 @@ CFDV_HD CFDV_INLINE void phase_contract_domain(FormShared<NDIM>& sh, int tid) {
         for (int i = 0; i < NDIM; i++) h += sl.dPhi[N][i] * sl.H[i * 3 + j][idx];
         G[1 + j] = wJ * h;
       }
-      if (NDIM == 2) {
-        double sx = 0.0;
-        for (int i = 0; i < NDIM; i++) sx += sl.X[i][idx];
-        G[NC - 1] = wJ * sl.Psi[N] * sx;
-      }
+      double sx = 0.0;
+      for (int i = 0; i < NDIM; i++) sx += sl.X[i][idx];
+      G[NC - 1] = wJ * sl.Psi[N] * sx;
       for (int M = 0; M < NNOD; M++) {
         double t = acc[M];
         for (int c = 0; c < NC; c++) t += sl.cM[c][M] * G[c];
@@ -859,17 +856,7 @@ CFDV_HD CFDV_INLINE void step_face_geom(const FormArgs& a, FormShared<NDIM>& sh,
   const int f = sh.faces[lf];
   const double* xf[NBN];
   for (int i = 0; i < NBN; i++) xf[i] = sh.nd[face_node(NDIM, f, i)].x;
-  double xl[4][3];
-  const double* H = (NDIM == 3 && sh.hnm >= 0) ? a.hnm + (size_t)sh.hnm * 64 : nullptr;
-  if (H) {
-    const double* xe[8];
-    for (int M = 0; M < 8; M++) xe[M] = sh.nd[M % T::NNOD].x;
-    hnm_face_nodes_3d(H, xe, f, xl);
-    for (int i = 0; i < NBN; i++) xf[i] = xl[i % 4];
-  }
   face_point_geom<NDIM>(a.gz, a.gw, xf, qf, sl.Phi, sl.dPhi, sl.en);
-  if constexpr (NDIM == 3)
-    if (H) hnm_face_phi_3d(H, f, sl.Phi);
   for (int m = 0; m < NBN; m++) {
     sl.cM[0][m] = sl.Phi[m];
     for (int j = 0; j < NDIM; j++) sl.cM[1 + j][m] = sl.dPhi[m][j];
@@ -877,7 +864,7 @@ CFDV_HD CFDV_INLINE void step_face_geom(const FormArgs& a, FormShared<NDIM>& sh,
 }
 
 // face step 2: viscosity and conductivity at the face point, stress zero, then the
-// boundary-condition edits of the state (eval1dboundary.h, eval2dboundary.h)
+// boundary-condition edits of the state (eval1dboundary.h)
 template <int NDIM>
 CFDV_HD CFDV_INLINE void step_face_edit(const FormArgs& a, FormShared<NDIM>& sh, int lf, int qf) {
   using T = FormTraits<NDIM>;
@@ -889,8 +876,7 @@ CFDV_HD CFDV_INLINE void step_face_edit(const FormArgs& a, FormShared<NDIM>& sh,
   fs.k = gas_k(a.gas, fs.mu);
   for (int i = 0; i < NDIM; i++)
     for (int j = 0; j < NDIM; j++) fs.tau[i][j] = 0;
-  if (NDIM == 2) edit_face_state_2d(code, fs, sh.nd[face_node(NDIM, f, 0)].x, sh.nd[face_node(NDIM, f, 1)].x, sl.en);
-  else edit_face_state_3d(code, fs, sl.en, a.gas.adiabatic);
+  edit_face_state_2d(code, fs, sh.nd[face_node(NDIM, f, 0)].x, sh.nd[face_node(NDIM, f, 1)].x, sl.en);
 }
 
 template <int NDIM>
@@ -982,6 +968,12 @@ CFDV_HD CFDV_INLINE void phase_write(const FormArgs& a, FormShared<NDIM>& sh, in
     for (int i = 0; i < 4; i++) a.s_out[(size_t)e * 4 + i] = sh.s[i];
 }
 
+}  // namespace cfdv
+
+#include "formation_hex.cuh"
+
+namespace cfdv {
+
 // ---- the element as a sequence of block-wide steps --------------------------------
 // Steps 0-9 form the domain integrals (step 9 leaves the element matrix in the shared
 // tile), then seven steps per boundary face (geometry, state sums, boundary edits,
@@ -993,38 +985,43 @@ constexpr int kFaceSteps = 7;
 
 template <int NDIM>
 CFDV_HD CFDV_INLINE int form_nsteps(const FormShared<NDIM>& sh) {
+  if constexpr (NDIM == 3) return hex_nsteps(sh);
   return kDomainSteps + kFaceSteps * sh.nfaces + 1;
 }
 
 template <int NDIM>
 CFDV_HD CFDV_INLINE void form_step(int k, const FormArgs& a, FormShared<NDIM>& sh, int e, int tid, int* bad) {
-  switch (k) {
-    case 0: step_load<NDIM>(a, sh, e, tid); return;
-    case 1: step_geom_jac<NDIM>(a, sh, tid); return;
-    case 2: step_geom_det<NDIM>(a, sh, tid); return;
-    case 3: step_dphi<NDIM>(sh, tid); return;
-    case 4: step_state<NDIM, false>(sh, 0, tid); return;
-    case 5: step_stress<NDIM>(a, sh, tid); return;
-    case 6: step_jacobians<NDIM, false>(a, sh, 0, tid); return;
-    case 7: step_coeffs<NDIM, false>(a, sh, tid); return;
-    case 8: step_hmat_rhs<NDIM, false>(a, sh, tid); return;
-    case 9: phase_contract_domain<NDIM>(sh, tid); return;
-    default: break;
-  }
-  const int f = k - kDomainSteps, nf = sh.nfaces;
-  if (f < kFaceSteps * nf) {
-    const int lf = f / kFaceSteps;
-    switch (f % kFaceSteps) {
-      case 0: step_face_geom<NDIM>(a, sh, lf, tid); return;
-      case 1: step_state<NDIM, true>(sh, lf, tid); return;
-      case 2: step_face_edit<NDIM>(a, sh, lf, tid); return;
-      case 3: step_jacobians<NDIM, true>(a, sh, lf, tid); return;
-      case 4: step_coeffs<NDIM, true>(a, sh, tid); return;
-      case 5: step_hmat_rhs<NDIM, true>(a, sh, tid); return;
-      default: phase_contract_face<NDIM>(sh, lf, tid); return;
+  if constexpr (NDIM == 3) {
+    hex_step(k, a, sh, e, tid, bad);
+  } else {
+    switch (k) {
+      case 0: step_load<NDIM>(a, sh, e, tid); return;
+      case 1: step_geom_jac<NDIM>(a, sh, tid); return;
+      case 2: step_geom_det<NDIM>(a, sh, tid); return;
+      case 3: step_dphi<NDIM>(sh, tid); return;
+      case 4: step_state<NDIM, false>(sh, 0, tid); return;
+      case 5: step_stress<NDIM>(a, sh, tid); return;
+      case 6: step_jacobians<NDIM, false>(a, sh, 0, tid); return;
+      case 7: step_coeffs<NDIM, false>(a, sh, tid); return;
+      case 8: step_hmat_rhs<NDIM, false>(a, sh, tid); return;
+      case 9: phase_contract_domain<NDIM>(sh, tid); return;
+      default: break;
     }
+    const int f = k - kDomainSteps, nf = sh.nfaces;
+    if (f < kFaceSteps * nf) {
+      const int lf = f / kFaceSteps;
+      switch (f % kFaceSteps) {
+        case 0: step_face_geom<NDIM>(a, sh, lf, tid); return;
+        case 1: step_state<NDIM, true>(sh, lf, tid); return;
+        case 2: step_face_edit<NDIM>(a, sh, lf, tid); return;
+        case 3: step_jacobians<NDIM, true>(a, sh, lf, tid); return;
+        case 4: step_coeffs<NDIM, true>(a, sh, tid); return;
+        case 5: step_hmat_rhs<NDIM, true>(a, sh, tid); return;
+        default: phase_contract_face<NDIM>(sh, lf, tid); return;
+      }
+    }
+    phase_write<NDIM>(a, sh, e, tid, bad);
   }
-  phase_write<NDIM>(a, sh, e, tid, bad);
 }
 
 }  // namespace cfdv
