@@ -10,6 +10,7 @@
 
 #include "context.h"
 #include "adjoint.cuh"
+#include "adjoint_tangent.cuh"
 #include "adjoint_warp.cuh"
 #include "kernels.h"
 
@@ -20,18 +21,7 @@ using cfdv::ctxi::fail;
 
 namespace cfdv {
 
-// forward mode (the JVP, a.mode 1): one thread per (element, row), the row's derivative along
-// the tangent (tU, t_dt, t_mach)
-template <int NDIM>
-__global__ void __launch_bounds__(128) functional_kernel(FunctionalArgs a) {
-  constexpr int KE = FormTraits<NDIM>::KE;
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int e = (int)(t / KE), k = (int)(t % KE);
-  if (e >= a.n_elements) return;
-  a.out[(size_t)e * KE + k] = element_functional<NDIM>(a, e, k).d;
-}
-
-// the collectives of warp_vjp: the warp's lanes; task_sync is the block's barrier
+// the collectives of warp_vjp and warp_jvp: the warp's lanes; task_sync is the block's barrier
 struct WarpLanes {
   __device__ __forceinline__ void sync() const { __syncwarp(); }
   __device__ __forceinline__ double sum(double v, int m) const { return v + __shfl_xor_sync(0xffffffffu, v, m); }
@@ -60,6 +50,30 @@ cudaError_t launch_vjp_warp(const FunctionalArgs& a, cudaStream_t st) {
   if (attr != cudaSuccess) return attr;
   const int per_block = WarpVjp<NDIM>::EPW * kVjpWarps;
   vjp_warp_kernel<NDIM><<<(unsigned)((a.n_elements + per_block - 1) / per_block), 32 * kVjpWarps, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
+// forward mode, one lane per Gauss point: d r_e along (tU, t_dt, t_mach); each of the block's
+// kJvpWarps warps takes 4 (hex8) or 8 (quad4) elements.  The dual state of a point is thread
+// local (255 registers and local memory), so more warps per block would not raise residency.
+constexpr int kJvpWarps = 4;
+template <int NDIM>
+__global__ void __launch_bounds__(32 * kJvpWarps) jvp_warp_kernel(FunctionalArgs a) {
+  extern __shared__ __align__(16) unsigned char jvp_smem[];
+  const int w = (int)threadIdx.x / 32;
+  WarpJvpShared<NDIM>& sh = reinterpret_cast<WarpJvpShared<NDIM>*>(jvp_smem)[w];
+  WarpLanes L;
+  warp_jvp<NDIM>(a, sh, ((int)blockIdx.x * kJvpWarps + w) * WarpJvp<NDIM>::EPW, (int)threadIdx.x % 32, L);
+}
+
+template <int NDIM>
+cudaError_t launch_jvp_warp(const FunctionalArgs& a, cudaStream_t st) {
+  const size_t smem = sizeof(WarpJvpShared<NDIM>) * kJvpWarps;
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(jvp_warp_kernel<NDIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (attr != cudaSuccess) return attr;
+  const int per_block = WarpJvp<NDIM>::EPW * kJvpWarps;
+  jvp_warp_kernel<NDIM><<<(unsigned)((a.n_elements + per_block - 1) / per_block), 32 * kJvpWarps, smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -159,16 +173,6 @@ FunctionalArgs functional_args(cfdv_ctx* c, double dt) {
   return a;
 }
 
-cudaError_t launch_functional(cfdv_ctx* c, const FunctionalArgs& a) {
-  if (a.mode != 1) return cudaErrorInvalidValue;  // the VJP runs through vjp_warp_kernel
-  const long threads = (long)c->n_elements * c->Ke;
-  const int grid = (int)((threads + kThreadsFn - 1) / kThreadsFn);
-  if (c->ndim == 2) functional_kernel<2><<<grid, kThreadsFn, 0, c->st>>>(a);
-  else functional_kernel<3><<<grid, kThreadsFn, 0, c->st>>>(a);
-  c->launches++;
-  return cudaGetLastError();
-}
-
 // g = (dr/dU)^T w as a node vector (gather of the element rows), g_dt, g_mach; U, dt current
 int vjp_device(cfdv_ctx* c, double dt, const double* d_w, const double* d_du, double* d_g, double* g_dt,
                double* g_mach, double* d_val) {
@@ -200,13 +204,13 @@ int jvp_device(cfdv_ctx* c, double dt, const double* d_du, const double* d_tU, d
   int rc = ensure_adjoint_buffers(c);
   if (rc) return rc;
   FunctionalArgs a = functional_args(c, dt);
-  a.mode = 1;
   a.dU = d_du;
   a.tU = d_tU;
   a.t_dt = t_dt;
   a.t_mach = t_mach;
   a.out = c->d_adj_e;
-  CK(launch_functional(c, a));
+  CK(c->ndim == 2 ? launch_jvp_warp<2>(a, c->st) : launch_jvp_warp<3>(a, c->st));
+  c->launches++;
   CK(launch_compose_rhs(ebe_of(c), a.out, d_dr, c->d_pa, c->st));
   c->launches++;
   return CFDV_OK;
