@@ -245,7 +245,8 @@ int ensure_krylov(cfdv_ctx* c, int m) {
   if (m <= 0 || m > 255) return fail(c, CFDV_ERR_ARG, "gmres: m must be in [1, 255]");
   if (m <= c->m_cap) return CFDV_OK;
   int rc;
-  if ((rc = dalloc(c, &c->d_V, (size_t)(m + 1) * c->n_dof)) || (rc = dalloc(c, &c->d_H, (size_t)(m + 1) * m + 8)) ||
+  const size_t ldv = ((size_t)c->n_dof + 1) / 2 * 2;  // the persistent solve's vector stride
+  if ((rc = dalloc(c, &c->d_V, (size_t)(m + 1) * ldv)) || (rc = dalloc(c, &c->d_H, (size_t)(m + 1) * m + 8)) ||
       (rc = dalloc(c, &c->d_y, (size_t)m + 1)))
     return rc;
   c->m_cap = m;
@@ -565,7 +566,7 @@ int cfdv::ctxi::solve_launch(cfdv_ctx* c, const cfdv_gmres_opts* o, const double
   a.rtol = o->rtol;
   a.conn = c->d_conn; a.csr_ptr = c->d_csr_ptr; a.csr_idx = c->d_csr_idx;
   a.R64 = c->d_R64; a.R32 = c->d_R32; a.Y64 = c->d_Y64; a.Y32 = c->d_Y32;
-  a.b = c->d_b; a.du = c->d_du; a.V = c->d_V; a.W = c->d_W; a.part0 = c->d_pa; a.part1 = c->d_pb;
+  a.b = c->d_b; a.du = c->d_du; a.V = c->d_V; a.ldv = ((size_t)c->n_dof + 1) / 2 * 2; a.W = c->d_W; a.part0 = c->d_pa; a.part1 = c->d_pb;
   // A^T: transpose every element block in place (restored after the launch), so the kernel's
   // coalesced row loads stream R_e^T and the block Jacobi inverse is that of A^T
   float* r32 = c->have32 ? c->d_R32 : nullptr;

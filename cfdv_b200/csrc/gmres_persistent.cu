@@ -188,27 +188,32 @@ constexpr int kRingStages = 3;
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
+// mbarriers by shared address, and by pointer
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) { mbar_arrive(smem_addr(bar)); }
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+  mbar_expect_tx(smem_addr(bar), bytes);
 }
-__device__ __forceinline__ bool mbar_test(unsigned long long* bar, unsigned parity) {
+__device__ __forceinline__ bool mbar_test(unsigned bar, unsigned parity) {
   unsigned done;
   asm volatile(
       "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
       : "=r"(done)
-      : "r"(smem_addr(bar)), "r"(parity)
+      : "r"(bar), "r"(parity)
       : "memory");
   return done != 0;
 }
 // wait for the phase of `parity` to complete, at most kWaitNs, and give up early when another
 // block has set the launch's failure bit; false: the launch is failing (bit set here if not yet)
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, const Barrier& b) {
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, const Barrier& b) {
   if (mbar_test(bar, parity)) return true;
   const unsigned long long t0 = now_ns();
   for (unsigned polls = 1;; polls++) {
@@ -225,12 +230,15 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
     }
   }
 }
-__device__ __forceinline__ void bulk_to_shared(void* dst, const void* src, unsigned bytes, unsigned long long* bar,
+__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, const Barrier& b) {
+  return mbar_wait(smem_addr(bar), parity, b);
+}
+__device__ __forceinline__ void bulk_to_shared(unsigned dst, const void* src, unsigned bytes, unsigned bar,
                                                unsigned long long policy) {
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
-          smem_addr(dst)),
-      "l"(src), "r"(bytes), "r"(smem_addr(bar)), "l"(policy)
+          dst),
+      "l"(src), "r"(bytes), "r"(bar), "l"(policy)
       : "memory");
 }
 
@@ -293,7 +301,8 @@ __device__ __noinline__ void elem_pass_ring(const TM* __restrict__ R, const int*
         const int es = e0 + t * SE, ne = min(SE, e1 - es);
         const unsigned bytes = (unsigned)ne * EB;
         mbar_expect_tx(rv.full + sl, bytes);
-        bulk_to_shared(rv.buf + (size_t)sl * stage_bytes, R + (size_t)es * KE * KE, bytes, rv.full + sl, policy);
+        bulk_to_shared(smem_addr(rv.buf + (size_t)sl * stage_bytes), R + (size_t)es * KE * KE, bytes,
+                       smem_addr(rv.full + sl), policy);
         issued = t + 1;
       }
       // copies still in flight land before the pass ends (the consumers wait for them too;
@@ -343,6 +352,252 @@ __device__ __noinline__ void elem_pass_ring(const TM* __restrict__ R, const int*
     }
   }
   ring_t += T;
+}
+
+// ---- streamed basis through a shared-memory ring -------------------------------------------
+// The Gram-Schmidt passes of a streamed (not resident) basis read j vectors per pass.  A block's
+// slice is cut into chunks of K unknowns per consumer thread (K = 1 or 2), one ring stage is the
+// chunk of 4 (K = 1) or 2 (K = 2) vectors, and one producer thread fills the stages by bulk copies
+// while the other warps consume them, each thread keeping its unknowns of the chunk in registers.
+// The copies in flight depend on the ring alone, not on the loads that a 64-register thread can
+// have outstanding.  A stage costs about 0.4 us of waits and arrivals whatever its size (slope of a
+// pass over stages of 7.6 and of 15 KB), so a stage is as large as leaves the ring about five.
+// Ramp 128x64x32, mixed: dots 2.47 -> 1.45 ms and pass B 3.49 -> 1.40 ms a solve.
+constexpr int kGsLanes = kThreads - 32;  // consumer threads
+constexpr int kGsMaxSlots = 8, kGsMinSlots = 2;
+
+// unknowns per consumer thread and chunk length (even: bulk copies move multiples of 16 bytes) of
+// S unknowns a block: the choice with fewer thread-iterations, the larger stage on a tie
+__host__ __device__ constexpr int gs_chunks(int S, int K) { return (S + K * kGsLanes - 1) / (K * kGsLanes); }
+__host__ __device__ constexpr int gs_k(int S) { return 2 * gs_chunks(S, 2) <= gs_chunks(S, 1) ? 2 : 1; }
+__host__ __device__ constexpr int gs_chunk(int S) {
+  const int nch = gs_chunks(S, gs_k(S));
+  return ((S + nch - 1) / nch + 1) / 2 * 2;
+}
+__host__ __device__ constexpr int gs_group(int K) { return K == 1 ? 4 : 2; }  // vectors per stage
+__host__ __device__ constexpr size_t gs_slot_bytes(int S) {
+  return ((size_t)gs_group(gs_k(S)) * gs_chunk(S) * 8 + 127) / 128 * 128;
+}
+
+struct GsRing {
+  unsigned buf, full, empty;  // shared addresses: slots of slot_bytes; per slot a barrier for the producer's
+                              // arrival and the copies' bytes, and one for an arrival per consumer warp
+  unsigned slots, slot_bytes;
+  const double* V;            // own slice of basis vector 0; vector i at V + i * ld
+  size_t ld;
+  int ns, C;                  // own unknowns, chunk length
+  __device__ __forceinline__ int chunks() const { return (ns + C - 1) / C; }
+};
+// position in the ring: the slot of the next stage and how often the ring has been filled
+struct GsPos {
+  unsigned slot, fill;
+  __device__ __forceinline__ void next(const GsRing& r) {
+    if (++slot == r.slots) {
+      slot = 0;
+      fill++;
+    }
+  }
+  __device__ __forceinline__ void advance(const GsRing& r, unsigned stages) {
+    const unsigned t = slot + stages;
+    fill += t / r.slots;
+    slot = t % r.slots;
+  }
+};
+__device__ __forceinline__ double lds_f64(unsigned addr) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(addr));
+  return v;
+}
+
+// producer (one thread): vectors 0 .. j-1 of every chunk, G to a stage, chunks upwards or downwards
+template <int G>
+__device__ __forceinline__ void gs_produce(const GsRing& r, int j, bool down, GsPos p, const Barrier& bar) {
+  unsigned long long policy;
+  asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
+  const int nch = r.chunks();
+  const GsPos first = p;
+  int issued = 0;
+  bool ok = true;
+  for (int cc = 0; cc < nch && ok; cc++) {
+    const int c = down ? nch - 1 - cc : cc, n = min(r.C, r.ns - c * r.C);
+    const unsigned bytes = (unsigned)(n + (n & 1)) * 8u;  // an odd tail: the vectors' stride has room for one more
+    const double* src = r.V + (size_t)c * r.C;
+    for (int i = 0; i < j; i += G) {
+      if (p.fill >= 1 && !mbar_wait(r.empty + 8u * p.slot, (p.fill - 1) & 1u, bar)) { ok = false; break; }
+      const int nv = min(G, j - i);
+      mbar_expect_tx(r.full + 8u * p.slot, (unsigned)nv * bytes);
+      for (int v = 0; v < nv; v++)
+        bulk_to_shared(r.buf + p.slot * r.slot_bytes + (unsigned)(v * r.C) * 8u, src + (size_t)(i + v) * r.ld, bytes,
+                       r.full + 8u * p.slot, policy);
+      p.next(r);
+      issued++;
+    }
+  }
+  // copies still in flight land before the pass ends
+  const int last = min(issued, (int)r.slots);
+  p = first;
+  p.advance(r, (unsigned)(issued - last));
+  for (int q = 0; q < last; q++, p.next(r)) mbar_wait(r.full + 8u * p.slot, p.fill & 1u, bar);
+}
+
+// Consumer side of the dots: redw[i] = <q_i, u> and, with w, redw[j + i] = <q_i, w> over the
+// warp's unknowns (u: own slice of vector j), then <u,u> and with w <u,w>, <w,w>.  A warp owns 32 K
+// consecutive entries of a chunk.  The stage's G vectors against u and w are small dense products,
+// on the FP64 matrix instruction (m8n8k4): row b G + v is vector v at the entries of block b,
+// column 2 b + {0, 1} is u and w at block b (8 / G blocks of 4 entries a product), so the sums of
+// vector v stand where the row's block is the column's and 2 (G = 2) or 1 (G = 4) exchanges add
+// them up.  Summing each vector's two products over the lanes by shuffles took 6.2 us where this
+// takes 5.8 for 16 vectors of 141k unknowns (in L2), and 31.4 against 30.1 for 1.38M (at the copy
+// peak).
+template <int K>
+__device__ __forceinline__ void gs_dots(const GsRing& r, int j, const double* w, GsPos p, double* redw,
+                                        const Barrier& bar) {
+  constexpr int G = gs_group(K), NB = 8 / G, T = 32 * K / (4 * NB);  // T products a stage
+  const int lane = threadIdx.x & 31, nch = r.chunks();
+  const int e0 = ((int)threadIdx.x / 32 - 1) * 32 * K;  // the warp's entries of a chunk
+  const int row = lane >> 2, k4 = lane & 3;
+  const double* u = r.V + (size_t)j * r.ld;
+  const int nt = w ? 2 * j + 3 : j + 1;
+  for (int k = lane; k < nt; k += 32) redw[k] = 0.0;
+  __syncwarp();
+  // B operand of product t: u (even row) or w (odd row) at block row / 2
+  const double* src = (row & 1) ? w : u;
+  const bool have = (row >> 1) < NB && src != nullptr;
+  double nx[T];
+  auto fetch = [&](int c) {
+#pragma unroll
+    for (int t = 0; t < T; t++) {
+      const int e = e0 + t * 4 * NB + (row >> 1) * 4 + k4;
+      nx[t] = (have && c < nch && e < min(r.C, r.ns - c * r.C)) ? __ldcg(src + c * r.C + e) : 0.0;
+    }
+  };
+  double own2 = 0.0, cross = 0.0;
+  fetch(0);
+  for (int c = 0; c < nch; c++) {
+    const int n = min(r.C, r.ns - c * r.C);
+    double x[T];
+    unsigned ad[T];
+#pragma unroll
+    for (int t = 0; t < T; t++) {
+      x[t] = nx[t];
+      own2 += x[t] * x[t];
+      cross += x[t] * __shfl_xor_sync(0xffffffffu, x[t], 4);
+      // A operand: vector row % G at block row / G (past the chunk's end any entry: x is zero there)
+      ad[t] = (unsigned)((row % G) * r.C + min(e0 + t * 4 * NB + (row / G) * 4 + k4, n - 1)) * 8u;
+    }
+    fetch(c + 1);
+    for (int i0 = 0; i0 < j; i0 += G) {
+      if (!mbar_wait(r.full + 8u * p.slot, p.fill & 1u, bar)) return;
+      const unsigned b = r.buf + p.slot * r.slot_bytes;
+      double q[T], s0 = 0.0, s1 = 0.0;
+#pragma unroll
+      for (int t = 0; t < T; t++) q[t] = lds_f64(b + ad[t]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(r.empty + 8u * p.slot);
+      p.next(r);
+#pragma unroll
+      for (int t = 0; t < T; t++)
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                     : "+d"(s0), "+d"(s1)
+                     : "d"(q[t]), "d"(x[t]));
+      if constexpr (G == 2) {
+        s0 += __shfl_xor_sync(0xffffffffu, s0, 9);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, 9);
+        s0 += __shfl_xor_sync(0xffffffffu, s0, 18);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, 18);
+      } else {
+        s0 += __shfl_xor_sync(0xffffffffu, s0, 17);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, 17);
+      }
+      if (k4 == 0 && row < G && i0 + row < j) {  // block 0's lane of vector row
+        redw[i0 + row] += s0;
+        if (w) redw[j + i0 + row] += s1;
+      }
+    }
+  }
+  const double uu = xor_sum((row & 1) ? 0.0 : own2), ww = xor_sum((row & 1) ? own2 : 0.0),
+               uw = xor_sum((row & 1) ? 0.0 : cross);
+  if (lane == 0) {
+    const int s0 = w ? 2 * j : j;
+    redw[s0] = uu;
+    if (w) {
+      redw[s0 + 1] = uw;
+      redw[s0 + 2] = ww;
+    }
+  }
+}
+
+// x / d with the reciprocal of d at hand: one Newton correction of the quotient (Markstein's
+// final step) gives the correctly rounded quotient but for rare last-bit cases, in 3 operations;
+// the compiled division takes about 35 instructions, 3 to 8 us a pass B of 1.38M unknowns.
+// rd not a normal number (d tiny or huge): the division itself.
+struct Divisor {
+  double d, rd;
+  bool fast;
+  __device__ __forceinline__ explicit Divisor(double v) : d(v), rd(1.0 / v), fast(fabs(rd) >= 1e-290 && fabs(rd) <= 1e290) {}
+  __device__ __forceinline__ double operator()(double x) const {
+    if (!fast) return x / d;
+    const double q = x * rd;
+    return fma(fma(-q, d, x), rd, q);
+  }
+};
+
+// Consumer side of pass B, chunks downwards: for every own unknown, finish(dl, u, w, su, sw) with
+// su = sum_i cu[i] q_i, sw = sum_i cw[i] q_i and u = own slice of vector j
+template <int K, class F>
+__device__ __forceinline__ void gs_pass_b(const GsRing& r, int j, const double* w, const double* cu, const double* cw,
+                                          GsPos p, const Barrier& bar, F finish) {
+  constexpr int G = gs_group(K);
+  const int ct = threadIdx.x - 32;
+  double nu[K], nw[K];  // the next chunk's u and w
+  auto fetch = [&](int c) {
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const int e = ct + k * kGsLanes;
+      const bool in = c >= 0 && e < min(r.C, r.ns - c * r.C);
+      nu[k] = in ? __ldcg(r.V + (size_t)j * r.ld + c * r.C + e) : 0.0;
+      nw[k] = in ? __ldcg(w + c * r.C + e) : 0.0;
+    }
+  };
+  fetch(r.chunks() - 1);
+  for (int c = r.chunks() - 1; c >= 0; c--) {
+    const int n = min(r.C, r.ns - c * r.C);
+    double su[K], sw[K], ud[K], wd[K];
+    unsigned x[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      su[k] = sw[k] = 0.0;
+      ud[k] = nu[k];
+      wd[k] = nw[k];
+      x[k] = (unsigned)min(ct + k * kGsLanes, n - 1) * 8u;
+    }
+    fetch(c - 1);
+    for (int i0 = 0; i0 < j; i0 += G) {
+      if (!mbar_wait(r.full + 8u * p.slot, p.fill & 1u, bar)) return;
+      const unsigned b = r.buf + p.slot * r.slot_bytes;
+      double v[G][K];
+#pragma unroll
+      for (int q = 0; q < G; q++)
+#pragma unroll
+        for (int k = 0; k < K; k++) v[q][k] = i0 + q < j ? lds_f64(b + (unsigned)(q * r.C) * 8u + x[k]) : 0.0;
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) mbar_arrive(r.empty + 8u * p.slot);
+      p.next(r);
+#pragma unroll
+      for (int q = 0; q < G; q++)
+        if (i0 + q < j) {
+          const double hu = cu[i0 + q], hw = cw[i0 + q];
+#pragma unroll
+          for (int k = 0; k < K; k++) {
+            su[k] += hu * v[q][k];
+            sw[k] += hw * v[q][k];
+          }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if (ct + k * kGsLanes < n) finish(c * r.C + ct + k * kGsLanes, ud[k], wd[k], su[k], sw[k]);
+  }
 }
 
 // Element pass Y_e = R_e x_e, thread (le, i) owning row i of element le.
@@ -509,26 +764,66 @@ size_t persistent_dyn_doubles(int m, int S, bool resident, size_t ring_stage_byt
   return base + (resident ? (size_t)(m + 2) * S : (size_t)kWarps * kSlots);
 }
 
+// nodes per block: an even number of unknowns, so that every block's slice of a basis vector
+// starts on 16 bytes
+template <int NEQ>
+__host__ __device__ constexpr int own_nodes(int n_nodes, int blocks) {
+  const int pn = (n_nodes + blocks - 1) / blocks;
+  return NEQ % 2 ? pn + (pn & 1) : pn;
+}
+
 template <int KE, int NEQ, int NNOD, typename TR, bool RES>
 __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(PersistentArgs a) {
   extern __shared__ __align__(16) double dyn[];
   const int nb = gridDim.x, tid = threadIdx.x, bid = blockIdx.x, lane = tid & 31, wid = tid >> 5;
   const int n = a.n_dof, m = a.m;
   // own unknowns [lo, lo + ns): whole nodes, S per block
-  const int pn = (n / NEQ + nb - 1) / nb, S = pn * NEQ;
+  const int pn = own_nodes<NEQ>(n / NEQ, nb), S = pn * NEQ;
   const int lo = min(n, bid * S), ns = min(n, lo + S) - lo;
+  const size_t ldv = a.ldv;  // stride of the basis vectors (even)
   Barrier bar{a.bar_count, a.err, 0u};
   // one tile area for both products (FP64 restart residual, TR Arnoldi products)
   double* tile64 = dyn;
   TR* tileR = reinterpret_cast<TR*>(dyn);
   auto* first = reinterpret_cast<int (*)[kThreads]>(dyn + (size_t)ElemGroups<KE>::TILES);
-  // 3D with FP32 products (the mixed form): every element pass of the launch, the FP64 restart
-  // residuals included, streams its matrices through the shared-memory ring.  The FP64 form keeps
-  // the direct pass: measured, the ring made its whole solve slower (see the element pass notes).
-  const bool use_ring = KE == 40 && !RES && sizeof(TR) == 4 && a.ring_stage_bytes > 0;
+  // 3D with a streamed basis: every element pass of the launch streams its matrices through the
+  // shared-memory ring.  Loads in waves through L1 were as fast for the FP64 form (149k elements:
+  // 14.8 ms of element passes against 12.4, but shorter phases between) only while L1 had the
+  // shared memory that the basis's ring now takes: 20.1 ms a solve with them, 18.4 with the ring.
+  const bool use_ring = KE == 40 && !RES && a.ring_stage_bytes > 0;
   unsigned ring_t = 0;
   if (use_ring) ring_init(a.ring_stage_bytes);  // visible after the first grid barrier
   else elem_first<KE, NEQ, NNOD>(a.conn, a.n_elements, first);  // each thread reads its own entries
+  // 3D streamed basis (DCGS2): the ring of the Gram-Schmidt passes lies over the element ring's
+  // stages (the two are never in use together), or behind the other arrays.  In 2D a streamed
+  // basis stays in L2 with the matrices and the plain loops were as fast (391x203 quads: 2.37 ms
+  // a solve for both passes, 2.36 with the ring), while the ring's shared memory, taken from L1,
+  // slowed the element pass from 1.33 to 1.65 ms.
+  constexpr bool kGs = KE == 40 && !RES;
+  __shared__ unsigned long long gs_bar[2 * kGsMaxSlots];
+  GsRing gs;
+  GsPos gs_p{0u, 0u};
+  if constexpr (kGs) {
+    if (a.gs_bytes > 0) {
+      gs.slot_bytes = (unsigned)gs_slot_bytes(S);
+      gs.slots = min((unsigned)kGsMaxSlots, (unsigned)(a.gs_bytes / gs_slot_bytes(S)));
+      gs.buf = smem_addr(dyn) + (unsigned)a.gs_offset;
+      gs.full = smem_addr(gs_bar);
+      gs.empty = smem_addr(gs_bar + kGsMaxSlots);
+      gs.V = a.V + lo;
+      gs.ld = ldv;
+      gs.ns = ns;
+      gs.C = gs_chunk(S);
+      if (tid == 0) {
+        for (unsigned sl = 0; sl < gs.slots; sl++) {
+          mbar_init(gs_bar + sl, 1);
+          mbar_init(gs_bar + kGsMaxSlots + sl, kWarps - 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
+    }
+  }
   __shared__ double hs1[kSlots], hs2[kMaxBasis], sc[4];
   __shared__ int s_stop;
   double* g = dyn + (use_ring ? ring_total_bytes(a.ring_stage_bytes) / sizeof(double) : tile_doubles<KE>());  // Givens right-hand side
@@ -572,7 +867,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
   // own-slice accessors: basis entry i, w
   auto vld = [&](int i, int dl) -> double {
     if constexpr (RES) return sV[(size_t)i * S + dl];
-    else return __ldcg(V + (size_t)i * n + lo + dl);
+    else return __ldcg(V + (size_t)i * ldv + lo + dl);
   };
   auto wld = [&](int dl) -> double {
     if constexpr (RES) return sW[dl];
@@ -583,7 +878,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
     else W[lo + dl] = v;
   };
   auto vst = [&](int i, int dl, double v) {
-    V[(size_t)i * n + lo + dl] = v;  // the element pass gathers it when there is no preconditioner
+    V[(size_t)i * ldv + lo + dl] = v;  // the element pass gathers it when there is no preconditioner
     if constexpr (RES) sV[(size_t)i * S + dl] = v;
   };
 
@@ -720,6 +1015,11 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
     }
     return acc;
   };
+  // every thread: the stages of a pass over j vectors are behind it
+  auto gs_advance = [&](int j) {
+    const int G = gs_group(gs_k(S));
+    gs_p.advance(gs, (unsigned)((j + G - 1) / G * gs.chunks()));
+  };
   // DCGS2 pass A: partm[s][bid] over the own unknowns of, with u~ = slot j of V,
   //   s < j: <q_s, u~>;  with w: j <= s < 2j: <q_{s-j}, w>, 2j: <u~, u~>, 2j+1: <u~, w>,
   //   2j+2: <w, w>;  without w: j: <u~, u~>
@@ -738,7 +1038,24 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
         acc = xor_sum(acc);
         if (lane == 0) pm[(size_t)sl * kPartLd + bid] = acc;
       }
-    } else {  // streaming: each thread its own unknowns, four basis vectors per load batch
+    } else if constexpr (kGs) {  // the basis through the ring
+      __syncthreads();  // w written by other threads
+      const double* w = with_w ? W + lo : nullptr;
+      if (gs_k(S) == 1) {
+        if (tid == 0) gs_produce<gs_group(1)>(gs, j, false, gs_p, bar);
+        if (wid > 0) gs_dots<1>(gs, j, w, gs_p, red[wid], bar);
+      } else {
+        if (tid == 0) gs_produce<gs_group(2)>(gs, j, false, gs_p, bar);
+        if (wid > 0) gs_dots<2>(gs, j, w, gs_p, red[wid], bar);
+      }
+      gs_advance(j);
+      __syncthreads();
+      for (int sl = tid; sl < nt; sl += kThreads) {
+        double t = 0.0;
+        for (int k = 1; k < kWarps; k++) t += red[k][sl];
+        pm[(size_t)sl * kPartLd + bid] = t;
+      }
+    } else {  // 2D: each thread its own unknowns, four basis vectors per load batch
       for (int i0 = 0; i0 < j; i0 += 4) {
         double au[4] = {0.0, 0.0, 0.0, 0.0}, aw[4] = {0.0, 0.0, 0.0, 0.0};
         for (int dl = tid; dl < ns; dl += kThreads) {
@@ -797,6 +1114,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
   //   slot j+1 = u / sigma (sigma > 0), or u kept in w (sigma = 0); returns the share of ||u||^2
   // pass B by the first nthr threads of the block (the resident path's overlapped step)
   auto pass_b_part = [&](int j, double nu, double pj, double sigma, int nthr) {
+    const Divisor by_nu(nu), by_sigma(sigma);
     for (int dl = tid; dl < ns; dl += nthr) {
       double su = 0.0, sw = 0.0;
 #pragma unroll 4
@@ -805,28 +1123,44 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
         su += hs1[i] * q;
         sw += hs1[j + i] * q;
       }
-      const double qj = (vld(j, dl) - su) / nu;
+      const double qj = by_nu(vld(j, dl) - su);
       const double u = wld(dl) - sw - pj * qj;
       vst(j, dl, qj);
-      vst(j + 1, dl, u / sigma);
+      vst(j + 1, dl, by_sigma(u));
     }
   };
   auto pass_b = [&](int j, double nu, double pj, double sigma) -> double {
     double acc = 0.0;
-    for (int dl = tid; dl < ns; dl += kThreads) {
-      double su = 0.0, sw = 0.0;
-#pragma unroll 4
-      for (int i = 0; i < j; i++) {
-        const double q = vld(i, dl);
-        su += hs1[i] * q;
-        sw += hs1[j + i] * q;
-      }
-      const double qj = (vld(j, dl) - su) / nu;
-      const double u = wld(dl) - sw - pj * qj;
+    const Divisor by_nu(nu), by_sigma(sigma > 0.0 ? sigma : 1.0);
+    auto finish = [&](int dl, double u, double w, double su, double sw) {
+      const double qj = by_nu(u - su);
+      const double un = w - sw - pj * qj;
       vst(j, dl, qj);
-      if (sigma > 0.0) vst(j + 1, dl, u / sigma);
-      else wst(dl, u);
-      acc += u * u;
+      if (sigma > 0.0) vst(j + 1, dl, by_sigma(un));
+      else wst(dl, un);
+      acc += un * un;
+    };
+    if constexpr (!kGs) {
+      for (int dl = tid; dl < ns; dl += kThreads) {
+        double su = 0.0, sw = 0.0;
+#pragma unroll 4
+        for (int i = 0; i < j; i++) {
+          const double q = vld(i, dl);
+          su += hs1[i] * q;
+          sw += hs1[j + i] * q;
+        }
+        finish(dl, vld(j, dl), wld(dl), su, sw);
+      }
+    } else {
+      if (gs_k(S) == 1) {
+        if (tid == 0) gs_produce<gs_group(1)>(gs, j, true, gs_p, bar);
+        if (wid > 0) gs_pass_b<1>(gs, j, W + lo, hs1, hs1 + j, gs_p, bar, finish);
+      } else {
+        if (tid == 0) gs_produce<gs_group(2)>(gs, j, true, gs_p, bar);
+        if (wid > 0) gs_pass_b<2>(gs, j, W + lo, hs1, hs1 + j, gs_p, bar, finish);
+      }
+      gs_advance(j);
+      asm volatile("fence.proxy.async.global;" ::: "memory");  // the new slots, before bulk copies read them
     }
     return acc;
   };
@@ -944,6 +1278,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
       break;
     }
     for (int dl = tid; dl < ns; dl += kThreads) vst(0, dl, wld(dl) / beta);
+    if constexpr (kGs) asm volatile("fence.proxy.async.global;" ::: "memory");
     if (a.Dinv) precond_slice(0);
     for (int i = tid; i <= m; i += kThreads) g[i] = i == 0 ? beta : 0.0;
     if (!grid_sync(bar)) return;
@@ -957,7 +1292,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
       bool done = false;
       for (int j = 0; j < m && !done; j++) {
         pm = a.partm + (size_t)(j & 1) * kSlots * kPartLd;
-        elem_pass_op(a.Dinv ? a.Z : V + (size_t)j * n);  // A P u~_j
+        elem_pass_op(a.Dinv ? a.Z : V + (size_t)j * ldv);  // A P u~_j
         if (!sync_y()) return;
         node_pass(sizeof(TR) == 4, 0, nullptr);
         mv++;
@@ -1042,6 +1377,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
           sigma = sqrt(sum_partials(a.part0, nb));
           if (sigma > 0.0)
             for (int dl = tid; dl < ns; dl += kThreads) vst(j + 1, dl, wld(dl) / sigma);
+          if constexpr (kGs) asm volatile("fence.proxy.async.global;" ::: "memory");
         }
         passes += j + 2;
         if (!(sigma > 0.0)) {  // invariant subspace (or a non-finite norm): column j is final
@@ -1076,7 +1412,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
       }
     }
     for (int j = 0; j < m && !dcgs; j++) {
-      const double* xj = a.Dinv ? a.Z : V + (size_t)j * n;  // right preconditioning: A P v_j
+      const double* xj = a.Dinv ? a.Z : V + (size_t)j * ldv;  // right preconditioning: A P v_j
       elem_pass_op(xj);
       if (!grid_sync(bar)) return;
       const int nv = j + 1;
@@ -1119,7 +1455,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
         for (int i = 0; i <= j; i++) {
           const double h = sum_partials(pa, nb);
           if (tid == 0) col[i] = h;
-          const double* nx = (i < j) ? V + (size_t)(i + 1) * n : nullptr;
+          const double* nx = (i < j) ? V + (size_t)(i + 1) * ldv : nullptr;
           double acc = 0.0;
           for (int dl = tid; dl < ns; dl += kThreads) {
             const double wn = wld(dl) - h * vld(i, dl);
@@ -1226,7 +1562,7 @@ cudaError_t launch_one(const PersistentArgs& a, cudaStream_t st) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   const int blocks = sms < a.max_blocks ? sms : a.max_blocks;
-  const int pn = (a.n_dof / NEQ + blocks - 1) / blocks, S = pn * NEQ;
+  const int pn = own_nodes<NEQ>(a.n_dof / NEQ, blocks), S = pn * NEQ;
   const bool cgs = (a.orth == 0 || a.orth == 2 || a.orth == 3) && a.m + 2 <= kMaxBasis && a.partm != nullptr;
   cudaFuncAttributes fa;
   cudaError_t e = cudaFuncGetAttributes(&fa, gmres_persistent_kernel<KE, NEQ, NNOD, TR, true>);
@@ -1240,24 +1576,35 @@ cudaError_t launch_one(const PersistentArgs& a, cudaStream_t st) {
     return launch_cfg<KE, NEQ, NNOD, TR, true>(a, blocks, res_bytes, 0, st);
   e = cudaFuncGetAttributes(&fa, gmres_persistent_kernel<KE, NEQ, NNOD, TR, false>);
   if (e != cudaSuccess) return e;
-  if (KE == 40 && a.ring && sizeof(TR) == 4) {
+  const bool dcgs = KE == 40 && cgs && a.orth != 0;  // the basis through the ring
+  const size_t slot = gs_slot_bytes(S);
+  if (KE == 40 && a.ring) {
     // 3D: the largest ring stage (a multiple of one FP64 element matrix, at most 4 of them) that
     // fits beside the rest; stages hold 4 FP64 or 8 FP32 element matrices at m <= 50
     constexpr size_t kElem64 = (size_t)KE * KE * sizeof(double);
     for (size_t se = 4; se >= 1; se--) {
       const size_t ring_bytes = sizeof(double) * persistent_dyn_doubles<KE>(a.m, S, false, se * kElem64);
+      if (dcgs && ring_xbuf_offset(se * kElem64) < kGsMinSlots * slot) break;  // the basis ring lies over the stages
       if (fa.sharedSizeBytes + ring_bytes <= (size_t)optin) {
         PersistentArgs ar = a;
         ar.ring_stage_bytes = (int)(se * kElem64);
+        ar.gs_offset = 0;
+        ar.gs_bytes = dcgs ? ring_xbuf_offset(se * kElem64) : 0;
         return launch_cfg<KE, NEQ, NNOD, TR, false>(ar, blocks, ring_bytes, 0, st);
       }
     }
   }
-  const size_t str_bytes = sizeof(double) * persistent_dyn_doubles<KE>(a.m, S, false);
-  if (fa.sharedSizeBytes + str_bytes > (size_t)optin) return cudaErrorInvalidValue;  // m too large
+  const size_t str_bytes = (sizeof(double) * persistent_dyn_doubles<KE>(a.m, S, false) + 127) / 128 * 128;
+  if (fa.sharedSizeBytes + str_bytes + (dcgs ? kGsMinSlots * slot : 0) > (size_t)optin) return cudaErrorInvalidValue;  // m too large
   PersistentArgs ad = a;
   ad.ring_stage_bytes = 0;
-  return launch_cfg<KE, NEQ, NNOD, TR, false>(ad, blocks, str_bytes, 0, st);
+  ad.gs_offset = str_bytes;
+  ad.gs_bytes = 0;
+  if (dcgs) {
+    const size_t most = ((size_t)optin - fa.sharedSizeBytes - str_bytes) / slot;
+    ad.gs_bytes = slot * (most < 4 ? most : 4);
+  }
+  return launch_cfg<KE, NEQ, NNOD, TR, false>(ad, blocks, str_bytes + ad.gs_bytes, 0, st);
 }
 
 cudaError_t launch_dim(int ndim, int fp32, const PersistentArgs& a, cudaStream_t st) {

@@ -22,7 +22,8 @@ struct PersistentArgs {
   float* Y32;
   const double* b;
   double* du;                  // solution, starts at zero
-  double* V;                   // (m+1) Krylov vectors
+  double* V;                   // (m+1) Krylov vectors, 16-byte aligned
+  size_t ldv;                  // their stride: n_dof rounded up to even
   double* W;
   const double* Dinv;          // node-block Jacobi inverse (right preconditioning) or null
   double* Z;                   // preconditioned vector z_j = Dinv v_j
@@ -56,6 +57,7 @@ struct PersistentArgs {
   int ring;                    // 3D: 1 = stream the element matrices through the shared-memory ring
                                // (bulk copies under mbarriers), 0 = direct loads in waves
   int ring_stage_bytes;        // set at launch: bytes of one ring stage (0: direct loads)
+  size_t gs_offset, gs_bytes;  // set at launch: dynamic shared memory of the streamed basis's ring
 };
 
 int persistent_blocks();
