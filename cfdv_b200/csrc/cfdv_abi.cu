@@ -352,11 +352,12 @@ int compose_b(cfdv_ctx* c, double* bnorm) {
   return CFDV_OK;
 }
 
-int add_combination(cfdv_ctx* c, const std::vector<double>& y, int mm, bool pc = false) {
+// du += V y, V with stride ld (the preconditioned form: n_dof)
+int add_combination(cfdv_ctx* c, const std::vector<double>& y, int mm, size_t ld, bool pc = false) {
   for (int i = 0; i < mm; i++) c->h_pin[i] = y[i];
   CK(cudaMemcpyAsync(c->d_y, c->h_pin, sizeof(double) * mm, cudaMemcpyHostToDevice, c->st));
   if (pc) CK(launch_combine_precond(c->ndim, c->d_du, c->d_V, c->n_dof, c->d_y, mm, c->d_Dinv, c->n_nodes, c->st));
-  else CK(launch_combine(c->d_du, c->d_V, c->n_dof, c->d_y, mm, c->st));
+  else CK(launch_combine(c->d_du, c->d_V, c->n_dof, ld, c->d_y, mm, c->st));
   c->launches++;
   CK(cudaStreamSynchronize(c->st));  // h_pin is reused by the next read-back
   return CFDV_OK;
@@ -368,52 +369,190 @@ void push_est(cfdv_gmres_report* rep, double v) {
   rep->n_est++;
 }
 
-// The reference's GMRES (MPI_GMRES::iterate, MPI_GMRES.h:125-220) with its
-// estimate (rotate_and_check :696-730), rotation (:733-752) and back substitution
-// (:756-780) carried out on the host in the same arithmetic order.
+// stride of the persistent solve's basis vectors: even, so that each starts on 16 bytes
+size_t vec_stride(const cfdv_ctx* c) { return ((size_t)c->n_dof + 1) / 2 * 2; }
+
+// Arguments of a persistent solve of at most `restarts` cycles of m steps, without preconditioner,
+// and its scratch (allocated once, barrier counters cleared): est and gfinal lie next to each other
+int persistent_args(cfdv_ctx* c, int m, int restarts, int orth, double rtol, PersistentArgs* out) {
+  const int est_cap = std::max(1, m * std::max(restarts, 1));
+  const int gf_cap = std::max(1, restarts);
+  int rc;
+  // scratch: g, cs, sn, y (m+1 each) | est | gfinal | result(8)
+  const size_t need = 4 * (size_t)(m + 1) + est_cap + gf_cap + 8;
+  if (need > c->pers_cap) {
+    if ((rc = dalloc(c, &c->d_pers, need))) return rc;
+    c->pers_cap = need;
+  }
+  // stop, cycles, err, barrier count | a neighbour-sync flag per block, 32 apart
+  const size_t n_int = 32 + 32 * (size_t)persistent_max_blocks();
+  if (!c->d_pers_int && (rc = dalloc(c, &c->d_pers_int, n_int))) return rc;
+  CK(cudaMemsetAsync(c->d_pers_int, 0, sizeof(int) * n_int, c->st));
+  PersistentArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.n_dof = c->n_dof; a.n_elements = c->n_elements; a.m = m; a.max_restarts = restarts;
+  a.max_blocks = persistent_max_blocks();
+  a.orth = orth;
+  if (orth == 0 || orth == 2 || orth == 3) {  // two buffers of 128 partial slots
+    if (!c->d_pm && (rc = dalloc(c, &c->d_pm, (size_t)persistent_max_blocks() * 256))) return rc;
+    a.partm = c->d_pm;
+  }
+  a.rtol = rtol;
+  a.conn = c->d_conn; a.csr_ptr = c->d_csr_ptr; a.csr_idx = c->d_csr_idx;
+  a.R64 = c->d_R64; a.R32 = c->d_R32; a.Y64 = c->d_Y64; a.Y32 = c->d_Y32;
+  a.b = c->d_b; a.du = c->d_du; a.V = c->d_V; a.ldv = vec_stride(c); a.W = c->d_W;
+  a.part0 = c->d_pa; a.part1 = c->d_pb;
+  a.H = c->d_H;
+  double* p = c->d_pers;
+  a.g = p; a.cs = p + (m + 1); a.sn = p + 2 * (m + 1); a.y = p + 3 * (m + 1);
+  a.est = p + 4 * (m + 1); a.est_capacity = est_cap;
+  a.gfinal = a.est + est_cap; a.gfinal_capacity = gf_cap;
+  a.result = a.gfinal + gf_cap;
+  int* pi = c->d_pers_int;
+  a.stop = pi; a.out = pi + 1; a.err = pi + 2;
+  a.bar_count = (unsigned int*)(pi + 3);
+  a.nbr_ptr = c->d_nbr_ptr; a.nbr_idx = c->d_nbr_idx; a.nbr_blocks = c->nbr_blocks;
+  a.nbr_flag = (unsigned int*)(pi + 32);
+  a.max_valence = c->max_valence;
+  // 3D element pass through the shared-memory ring (default); CFDV_ELEM_RING=0 selects the
+  // direct-load pass (same products bit for bit), for comparison
+  static const int ring_env = [] {
+    const char* v = std::getenv("CFDV_ELEM_RING");
+    return (v && v[0] == '0') ? 0 : 1;
+  }();
+  a.ring = ring_env;
+  *out = a;
+  return CFDV_OK;
+}
+
+// the persistent launch, counted and (when profiling) timed
+int persistent_launch(cfdv_ctx* c, int fp32, const PersistentArgs& a) {
+  std::pair<cudaEvent_t, cudaEvent_t> ev{nullptr, nullptr};
+  if (c->prof) {
+    cudaEventCreate(&ev.first);
+    cudaEventCreate(&ev.second);
+    cudaEventRecord(ev.first, c->st);
+  }
+  CK(launch_gmres_persistent(c->ndim, fp32, a, c->st));
+  if (c->prof) {
+    cudaEventRecord(ev.second, c->st);
+    c->ev_solve.push_back(ev);
+  }
+  c->launches++;
+  return CFDV_OK;
+}
+
+// at least n doubles of pinned memory for a solve's history
+int grow_hist(cfdv_ctx* c, size_t n) {
+  if (n <= c->h_hist_cap) return CFDV_OK;
+  if (c->h_hist) cudaFreeHost(c->h_hist);
+  c->h_hist = nullptr;
+  c->h_hist_cap = 0;
+  CK(cudaMallocHost((void**)&c->h_hist, sizeof(double) * n));
+  c->h_hist_cap = n;
+  return CFDV_OK;
+}
+
+// One Arnoldi cycle of the reference-mode solve from the current du, by modified Gram-Schmidt with
+// one launch per pass: the unrotated Hessenberg columns into H, their number and ||r||.  The
+// persistent kernel's cycle (reference_cycle below) takes its place for m + 2 <= 64.
+int reference_cycle_host(cfdv_ctx* c, int m, double tol, std::vector<double>& h, int* k, double* mag_r,
+                         cfdv_gmres_report* rep) {
+  std::vector<double> hcol(m + 2);
+  int rc;
+  if ((rc = restart_residual(c, 0, c->d_du, mag_r, rep))) return rc;
+  double g = *mag_r;
+  *k = m;
+  for (int j = 0; j < m; j++) {
+    if ((rc = arnoldi_step(c, 0, m, j, hcol.data(), rep))) return rc;
+    for (int i = 0; i < j + 2; i++) h[(size_t)j * (m + 1) + i] = hcol[i];
+    // rotate_and_check's estimate: c, s from the unrotated columns, applied to g one after another
+    const double sn = hcol[j + 1] / std::sqrt(std::pow(hcol[j], 2) + std::pow(hcol[j + 1], 2));
+    g = -sn * g;
+    if (std::abs(g) < tol) { *k = j + 1; break; }
+  }
+  return CFDV_OK;
+}
+
+// The same cycle as one persistent launch (delayed CGS2): 3 grid-wide synchronisations a step
+// instead of a launch per Gram-Schmidt coefficient and a host round trip.  The host driver's step
+// (CFL, formation, solve, update, RMS) on the 32x32 cavity: 1.91 -> 0.47 ms; on 65,536 hexes (7
+// products) 3.45 -> 3.28 ms.
+int reference_cycle(cfdv_ctx* c, int m, bool x0_zero, std::vector<double>& h, int* k, double* mag_r, double* bnorm) {
+  PersistentArgs a;
+  int rc = persistent_args(c, m, 1, 2, 1.0E-9, &a);
+  if (rc) return rc;
+  a.x0_zero = x0_zero ? 1 : 0;
+  a.ref_cycle = 1;
+  if ((rc = persistent_launch(c, 0, a))) return rc;
+  const size_t nh = (size_t)(m + 1) * m;
+  if ((rc = grow_hist(c, nh))) return rc;
+  double* hp = c->h_pin + cfdv::ctxi::kPinSolve;
+  CK(cudaMemcpyAsync(hp, c->d_pers_int, sizeof(int) * 8, cudaMemcpyDeviceToHost, c->st));
+  CK(cudaMemcpyAsync(hp + 4, a.result, sizeof(double) * 8, cudaMemcpyDeviceToHost, c->st));
+  CK(cudaMemcpyAsync(c->h_hist, a.H, sizeof(double) * nh, cudaMemcpyDeviceToHost, c->st));
+  CK(cudaStreamSynchronize(c->st));
+  int hi[8];
+  std::memcpy(hi, hp, sizeof(hi));
+  if (hi[2] & 1) return fail(c, CFDV_ERR_CUDA, "persistent GMRES: grid barrier timed out");
+  if (hi[2] & 2) return fail(c, CFDV_ERR_NONFINITE, "persistent GMRES: non-finite residual");
+  const double* res = hp + 4;
+  *mag_r = res[0];
+  *k = (int)res[1];
+  *bnorm = res[6];
+  c->mv_launches += (long)res[3];
+  if (c->prof) {
+    const double n8 = 8.0 * c->n_dof;
+    c->solve_bytes += res[3] * ((double)c->n_elements * c->Ke * c->Ke * 8.0 + 2 * n8) + res[5] * n8;
+  }
+  for (int j = 0; j < *k; j++)
+    for (int i = 0; i < j + 2; i++) {
+      const double v = c->h_hist[(size_t)j * (m + 1) + i];
+      if (!std::isfinite(v)) return fail(c, CFDV_ERR_NONFINITE, "non-finite Hessenberg entry in GMRES");
+      h[(size_t)j * (m + 1) + i] = v;
+    }
+  return CFDV_OK;
+}
+
+// The reference's GMRES (MPI_GMRES::iterate, MPI_GMRES.h:125-220): the Arnoldi cycle on the device,
+// its estimate (rotate_and_check :696-730), rotation (:733-752) and back substitution (:756-780) on
+// the host in the same arithmetic order.
 int gmres_reference(cfdv_ctx* c, const cfdv_gmres_opts* o, cfdv_gmres_report* rep) {
   const int m = o->m;
   int rc = ensure_krylov(c, m);
   if (rc) return rc;
   CK(cudaMemsetAsync(c->d_du, 0, sizeof(double) * c->n_dof, c->st));
-  double bnorm;
-  if ((rc = compose_b(c, &bnorm))) return rc;
-  const double tol = bnorm * 1.0E-9;
-  if (rep) { rep->tol = tol; rep->bnorm = bnorm; }
-  std::vector<double> h((size_t)(m + 1) * m), g(m + 1), y(m), hcol(m + 2);
+  // one persistent launch per cycle where its arrays fit in shared memory (delayed CGS2's 64 slots)
+  const bool device = m + 2 <= 64;
+  double bnorm = 0.0;
+  if (device) {
+    CK(launch_compose_rhs(ebe_args(c), c->d_rhs, c->d_b, c->d_pa, c->st));
+    c->launches++;
+  } else if ((rc = compose_b(c, &bnorm))) {
+    return rc;
+  }
+  double tol = bnorm * 1.0E-9;
+  std::vector<double> h((size_t)(m + 1) * m), g(m + 1), y(m);
   auto H = [&](int i, int j) -> double& { return h[(size_t)j * (m + 1) + i]; };
+  if (o->restarts == 0 && device && (rc = compose_b(c, &bnorm))) return rc;
   for (int gloop = 0; gloop < o->restarts; gloop++) {
     std::fill(h.begin(), h.end(), 0.0);
     std::fill(g.begin(), g.end(), 0.0);
     std::fill(y.begin(), y.end(), 0.0);
     double mag_r;
-    if ((rc = restart_residual(c, 0, c->d_du, &mag_r, rep))) return rc;
-    g[0] = mag_r;
-    int mm = m;
-    for (int j = 0; j < m; j++) {
-      if ((rc = arnoldi_step(c, 0, m, j, hcol.data(), rep))) return rc;
-      for (int i = 0; i < j + 2; i++) H(i, j) = hcol[i];
-      // rotate_and_check(j+1): c, s from the unrotated h applied to a rotated copy
-      const int nn = j + 1;
-      std::vector<double> hh((size_t)(nn + 1) * nn), gg(nn + 1, 0.0);
-      auto HH = [&](int i, int jj) -> double& { return hh[(size_t)jj * (nn + 1) + i]; };
-      gg[0] = g[0];
-      for (int i = 0; i < nn + 1; i++)
-        for (int jj = 0; jj < nn; jj++) HH(i, jj) = H(i, jj);
-      for (int i = 0; i < nn; i++) {
-        const double mag = std::sqrt(std::pow(H(i, i), 2) + std::pow(H(i + 1, i), 2));
-        const double cs = H(i, i) / mag, sn = H(i + 1, i) / mag;
-        for (int jj = 0; jj < nn; jj++) {
-          const double h0 = HH(i, jj), h1 = HH(i + 1, jj);
-          HH(i, jj) = cs * h0 + sn * h1;
-          HH(i + 1, jj) = -sn * h0 + cs * h1;
-        }
-        gg[i + 1] = -sn * gg[i];
-        gg[i] = cs * gg[i];
-      }
-      push_est(rep, gg[nn]);
-      if (std::abs(gg[nn]) < tol) { mm = j + 1; break; }
+    int mm;
+    rc = device ? reference_cycle(c, m, gloop == 0, h, &mm, &mag_r, &bnorm)
+                : reference_cycle_host(c, m, tol, h, &mm, &mag_r, rep);
+    if (rc) return rc;
+    tol = bnorm * 1.0E-9;
+    if (device && rep) rep->n_matvec += 1 + mm;
+    // the estimates of the cycle: c, s from the unrotated columns
+    double est = mag_r;
+    for (int j = 0; j < mm; j++) {
+      est = -(H(j + 1, j) / std::sqrt(std::pow(H(j, j), 2) + std::pow(H(j + 1, j), 2))) * est;
+      push_est(rep, est);
     }
+    g[0] = mag_r;
     for (int i = 0; i < mm; i++) {  // rotate()
       const double mag = std::sqrt(std::pow(H(i, i), 2) + std::pow(H(i + 1, i), 2));
       const double cs = H(i, i) / mag, sn = H(i + 1, i) / mag;
@@ -432,9 +571,10 @@ int gmres_reference(cfdv_ctx* c, const cfdv_gmres_opts* o, cfdv_gmres_report* re
         if (i != j) y[j] -= H(i, j) * y[i];
       y[j] /= H(j, j);
     }
-    if ((rc = add_combination(c, y, mm))) return rc;
+    if ((rc = add_combination(c, y, mm, device ? vec_stride(c) : (size_t)c->n_dof))) return rc;
     if (rep) rep->n_restarts = gloop + 1;
   }
+  if (rep) { rep->tol = bnorm * 1.0E-9; rep->bnorm = bnorm; }
   return CFDV_OK;
 }
 
@@ -503,7 +643,7 @@ int gmres_correct(cfdv_ctx* c, const cfdv_gmres_opts* o, cfdv_gmres_report* rep)
       for (int jj = i + 1; jj < k; jj++) s -= H(i, jj) * y[jj];
       y[i] = s / H(i, i);
     }
-    if ((rc = add_combination(c, y, k, pc))) return rc;
+    if ((rc = add_combination(c, y, k, (size_t)c->n_dof, pc))) return rc;
     if (rep && rep->gfinal && gloop < rep->gfinal_capacity) rep->gfinal[gloop] = g[k];
     if (rep) rep->n_restarts = gloop + 1;
   }
@@ -530,17 +670,6 @@ int cfdv::ctxi::solve_launch(cfdv_ctx* c, const cfdv_gmres_opts* o, const double
   if (fp32 && !c->have32) return fail(c, CFDV_ERR_STATE, "mixed precision needs cfdv_form(..., CFDV_PREC_MIXED)");
   int rc = ensure_krylov(c, m);
   if (rc) return rc;
-  const int est_cap = std::max(1, m * std::max(o->restarts, 1));
-  const int gf_cap = std::max(1, o->restarts);
-  // scratch: g, cs, sn, y (m+1 each) | est | gfinal | result(8)
-  const size_t need = 4 * (size_t)(m + 1) + est_cap + gf_cap + 8;
-  if (need > c->pers_cap) {
-    if ((rc = dalloc(c, &c->d_pers, need))) return rc;
-    c->pers_cap = need;
-  }
-  // stop, cycles, err, barrier count | a neighbour-sync flag per block, 32 apart
-  const size_t n_int = 32 + 32 * (size_t)persistent_max_blocks();
-  if (!c->d_pers_int && (rc = dalloc(c, &c->d_pers_int, n_int))) return rc;
   if (!x0) CK(cudaMemsetAsync(c->d_du, 0, sizeof(double) * c->n_dof, c->st));
   else if (x0 != c->d_du)
     CK(cudaMemcpyAsync(c->d_du, x0, sizeof(double) * c->n_dof, cudaMemcpyDeviceToDevice, c->st));
@@ -553,20 +682,8 @@ int cfdv::ctxi::solve_launch(cfdv_ctx* c, const cfdv_gmres_opts* o, const double
     CK(launch_compose_rhs(ebe_args(c), c->d_rhs, c->d_b, c->d_pa, c->st));
     c->launches++;
   }
-  CK(cudaMemsetAsync(c->d_pers_int, 0, sizeof(int) * n_int, c->st));
   PersistentArgs a;
-  std::memset(&a, 0, sizeof(a));
-  a.n_dof = c->n_dof; a.n_elements = c->n_elements; a.m = m; a.max_restarts = o->restarts;
-  a.max_blocks = persistent_max_blocks();
-  a.orth = o->orth;
-  if (o->orth == 0 || o->orth == 2 || o->orth == 3) {  // two buffers of 128 partial slots
-    if (!c->d_pm && (rc = dalloc(c, &c->d_pm, (size_t)persistent_max_blocks() * 256))) return rc;
-    a.partm = c->d_pm;
-  }
-  a.rtol = o->rtol;
-  a.conn = c->d_conn; a.csr_ptr = c->d_csr_ptr; a.csr_idx = c->d_csr_idx;
-  a.R64 = c->d_R64; a.R32 = c->d_R32; a.Y64 = c->d_Y64; a.Y32 = c->d_Y32;
-  a.b = c->d_b; a.du = c->d_du; a.V = c->d_V; a.ldv = ((size_t)c->n_dof + 1) / 2 * 2; a.W = c->d_W; a.part0 = c->d_pa; a.part1 = c->d_pb;
+  if ((rc = persistent_args(c, m, o->restarts, o->orth, o->rtol, &a))) return rc;
   // A^T: transpose every element block in place (restored after the launch), so the kernel's
   // coalesced row loads stream R_e^T and the block Jacobi inverse is that of A^T
   float* r32 = c->have32 ? c->d_R32 : nullptr;
@@ -582,58 +699,22 @@ int cfdv::ctxi::solve_launch(cfdv_ctx* c, const cfdv_gmres_opts* o, const double
     a.Dinv = c->d_Dinv;
     a.Z = c->d_Z;
   }
-  a.H = c->d_H;
-  double* p = c->d_pers;
-  a.g = p; a.cs = p + (m + 1); a.sn = p + 2 * (m + 1); a.y = p + 3 * (m + 1);
-  a.est = p + 4 * (m + 1); a.est_capacity = est_cap;
-  a.gfinal = a.est + est_cap; a.gfinal_capacity = gf_cap;
-  a.result = a.gfinal + gf_cap;
-  int* pi = c->d_pers_int;
-  a.stop = pi; a.out = pi + 1; a.err = pi + 2;
-  a.bar_count = (unsigned int*)(pi + 3);
-  a.nbr_ptr = c->d_nbr_ptr; a.nbr_idx = c->d_nbr_idx; a.nbr_blocks = c->nbr_blocks;
-  a.nbr_flag = (unsigned int*)(pi + 32);
-  a.max_valence = c->max_valence;
-  // 3D element pass through the shared-memory ring (default); CFDV_ELEM_RING=0 selects the
-  // direct-load pass (same products bit for bit), for comparison
-  static const int ring_env = [] {
-    const char* v = std::getenv("CFDV_ELEM_RING");
-    return (v && v[0] == '0') ? 0 : 1;
-  }();
-  a.ring = ring_env;
-  std::pair<cudaEvent_t, cudaEvent_t> ev{nullptr, nullptr};
-  if (c->prof) {
-    cudaEventCreate(&ev.first);
-    cudaEventCreate(&ev.second);
-    cudaEventRecord(ev.first, c->st);
-  }
-  CK(launch_gmres_persistent(c->ndim, fp32, a, c->st));
-  if (c->prof) {
-    cudaEventRecord(ev.second, c->st);
-    c->ev_solve.push_back(ev);
-  }
-  c->launches++;
+  if ((rc = persistent_launch(c, fp32, a))) return rc;
   if (transpose == 1) {  // restore the blocks (kTransposeKeep leaves them transposed)
     CK(launch_transpose_blocks(c->Ke, c->d_R64, r32, c->n_elements, c->st));
     c->launches += r32 ? 2 : 1;
   }
   double* hp = c->h_pin + cfdv::ctxi::kPinSolve;
-  CK(cudaMemcpyAsync(hp, pi, sizeof(int) * 8, cudaMemcpyDeviceToHost, c->st));
+  CK(cudaMemcpyAsync(hp, c->d_pers_int, sizeof(int) * 8, cudaMemcpyDeviceToHost, c->st));
   CK(cudaMemcpyAsync(hp + 4, a.result, sizeof(double) * 8, cudaMemcpyDeviceToHost, c->st));
   // the residual history comes back with the results (est and gfinal are contiguous), so the
   // report needs no copy after the wait
-  const size_t nh = (size_t)est_cap + gf_cap;
-  if (nh > c->h_hist_cap) {
-    if (c->h_hist) cudaFreeHost(c->h_hist);
-    c->h_hist = nullptr;
-    c->h_hist_cap = 0;
-    CK(cudaMallocHost((void**)&c->h_hist, sizeof(double) * nh));
-    c->h_hist_cap = nh;
-  }
+  const size_t nh = (size_t)a.est_capacity + a.gfinal_capacity;
+  if ((rc = grow_hist(c, nh))) return rc;
   CK(cudaMemcpyAsync(c->h_hist, a.est, sizeof(double) * nh, cudaMemcpyDeviceToHost, c->st));
   L->h_est = c->h_hist;
-  L->h_gfinal = c->h_hist + est_cap;
-  L->est = a.est; L->gfinal = a.gfinal; L->est_cap = est_cap; L->gf_cap = gf_cap;
+  L->h_gfinal = c->h_hist + a.est_capacity;
+  L->est = a.est; L->gfinal = a.gfinal; L->est_cap = a.est_capacity; L->gf_cap = a.gfinal_capacity;
   L->err = a.err; L->fp32 = fp32;
   return CFDV_OK;
 }

@@ -1226,7 +1226,13 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
   // by one thread of every block; sets s_stop
   int total_est = 0;
   auto givens = [&](int j, double nrm) {
-    if (tid == kThreads - 1) {
+    if (tid == kThreads - 1 && a.ref_cycle) {
+      // the reference's estimate: c, s from the unrotated column (MPI_GMRES.h:696-730)
+      const double h = col[j], sn_j = nrm / sqrt(h * h + nrm * nrm);
+      g[j + 1] = -sn_j * g[j];
+      s_stop = (fabs(g[j + 1]) < atol || nrm == 0.0 || !(nrm == nrm)) ? 1 : 0;
+      if (bid == 0 && total_est < a.est_capacity) a.est[total_est] = g[j + 1];
+    } else if (tid == kThreads - 1) {
       double* Rj = tri + (size_t)j * (j + 1) / 2;
       double hi = col[0];
       for (int i = 0; i < j; i++) {
@@ -1255,25 +1261,30 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
 
   int mv = 0, mv64 = 0;
   long passes = 0;  // algorithmic DOF-vector passes of the orthogonalisation and combination
-  bool converged = bnorm == 0.0;  // b = 0: du = 0 is the solution
+  bool converged = bnorm == 0.0 && !a.ref_cycle;  // b = 0: du = 0 is the solution
   double beta = 0.0;
   for (int cycle = 0; cycle < a.max_restarts && !converged; cycle++) {
-    // r = b - A64 du, beta = ||r||
-    elem_pass64(a.du);
-    if (!grid_sync(bar)) return;
-    {
-      const double acc = block_sum(node_pass(false, 1, nullptr));
-      if (tid == 0) a.part0[bid] = acc;
+    // r = b - A64 du, beta = ||r||; from du = 0, r = b and beta = ||b||
+    if (cycle == 0 && a.x0_zero) {
+      for (int dl = tid; dl < ns; dl += kThreads) wst(dl, a.b[lo + dl]);
+      beta = bnorm;
+    } else {
+      elem_pass64(a.du);
+      if (!grid_sync(bar)) return;
+      {
+        const double acc = block_sum(node_pass(false, 1, nullptr));
+        if (tid == 0) a.part0[bid] = acc;
+      }
+      mv++;
+      mv64++;
+      if (!grid_sync(bar)) return;
+      beta = sqrt(sum_partials(a.part0, nb));
     }
-    mv++;
-    mv64++;
-    if (!grid_sync(bar)) return;
-    beta = sqrt(sum_partials(a.part0, nb));
     if (!(beta == beta)) {
       if (bid == 0 && tid == 0) atomicOr(a.err, 2);
       return;
     }
-    if (beta < atol) {
+    if (beta < atol && !a.ref_cycle) {
       converged = true;
       break;
     }
@@ -1382,7 +1393,8 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
         passes += j + 2;
         if (!(sigma > 0.0)) {  // invariant subspace (or a non-finite norm): column j is final
           __syncthreads();
-          for (int r = tid; r <= j; r += kThreads) col[r] = pend[r];
+          for (int r = tid; r <= j; r += kThreads) col[r] = Hf[(size_t)j * (m + 1) + r] = pend[r];
+          if (tid == 0) Hf[(size_t)j * (m + 1) + j + 1] = 0.0;
           __syncthreads();
           givens(j, 0.0);
           total_est++;
@@ -1404,7 +1416,9 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
         reduce_parts(m + 1, hs1);
         dcgs_scalars(m, false);
         const double nu = sc[0];
-        for (int r = tid; r < m; r += kThreads) col[r] = pend[r] + tpend * hs1[r];
+        for (int r = tid; r < m; r += kThreads)
+          col[r] = Hf[(size_t)(m - 1) * (m + 1) + r] = pend[r] + tpend * hs1[r];
+        if (tid == 0) Hf[(size_t)(m - 1) * (m + 1) + m] = tpend * nu;
         __syncthreads();
         givens(m - 1, tpend * nu);
         total_est++;
@@ -1478,6 +1492,23 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
       k = j + 1;
       if (!grid_sync(bar)) return;
       if (s_stop) break;
+    }
+    if (a.ref_cycle) {  // the host rotates the Hessenberg matrix and substitutes as the reference does
+      if (bid == 0) {
+        for (int t = tid; t < k * (m + 1); t += kThreads) a.H[t] = Hf[t];
+        if (tid == 0) {
+          a.out[0] = 1;
+          a.result[0] = beta;
+          a.result[1] = (double)k;
+          a.result[2] = (double)total_est;
+          a.result[3] = (double)mv;
+          a.result[4] = (double)mv64;
+          a.result[5] = (double)passes;
+          a.result[6] = bnorm;
+          a.result[7] = atol;
+        }
+      }
+      return;
     }
     // y from R y = g (column-oriented back substitution by one warp of every block)
     if (wid == 0) {

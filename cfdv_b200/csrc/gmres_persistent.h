@@ -21,7 +21,10 @@ struct PersistentArgs {
   double* Y64;
   float* Y32;
   const double* b;
-  double* du;                  // solution, starts at zero
+  double* du;                  // solution: the start, zero with x0_zero
+  int x0_zero;                 // 1: du is zero, so the first cycle's r is b and needs no product
+  int ref_cycle;               // 1: one Arnoldi cycle of the reference's GMRES: its estimate stops the
+                               // cycle, H (unrotated, column-major) and V are the result, du stays
   double* V;                   // (m+1) Krylov vectors, 16-byte aligned
   size_t ldv;                  // their stride: n_dof rounded up to even
   double* W;
@@ -40,7 +43,7 @@ struct PersistentArgs {
   int gfinal_capacity;
   int* stop;
   int* out;                    // [0] cycles run
-  double* result;              // [0] final ||r||, [1] converged, [2] estimates, [3] products,
+  double* result;              // [0] final ||r||, [1] converged (ref_cycle: columns), [2] estimates, [3] products,
                                // [4] FP64 products, [5] algorithmic vector passes, [6] ||b||,
                                // [7] the stopping threshold rtol ||b||
   unsigned int* bar_count;     // grid barrier arrivals, zero before launch

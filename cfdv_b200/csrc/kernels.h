@@ -105,8 +105,8 @@ cudaError_t launch_normalize(const double* w, int n, const double* pin, double* 
                              cudaStream_t st);
 // *out = sum(pin) (single value, for host read-back)
 cudaError_t launch_reduce(const double* pin, double* out, int do_sqrt, cudaStream_t st);
-// x += sum_i y_i V_i  (V column-major, ld = n), summed in i order per entry
-cudaError_t launch_combine(double* x, const double* V, int n, const double* y, int m, cudaStream_t st);
+// x += sum_i y_i V_i  (V column-major, stride ld), summed in i order per entry
+cudaError_t launch_combine(double* x, const double* V, int n, size_t ld, const double* y, int m, cudaStream_t st);
 // out[i] = (float) in[i]
 cudaError_t launch_to_float(const double* in, float* out, size_t n, cudaStream_t st);
 // transpose every element block of R64 and R32 (either may be null) in place; ke = 16 or 40

@@ -141,14 +141,14 @@ __global__ void reduce_kernel(const double* __restrict__ pin, double* out, int d
   if (threadIdx.x == 0) out[0] = do_sqrt ? sqrt(s) : s;
 }
 
-__global__ void __launch_bounds__(kRedThreads) combine_kernel(double* x, const double* __restrict__ V, int n,
+__global__ void __launch_bounds__(kRedThreads) combine_kernel(double* x, const double* __restrict__ V, int n, size_t ld,
                                                               const double* __restrict__ y, int m) {
   __shared__ double ys[256];
   for (int i = threadIdx.x; i < m; i += blockDim.x) ys[i] = y[i];
   __syncthreads();
   for (int d = blockIdx.x * blockDim.x + threadIdx.x; d < n; d += gridDim.x * blockDim.x) {
     double z = 0.0;
-    for (int i = 0; i < m; i++) z += ys[i] * V[(size_t)i * n + d];
+    for (int i = 0; i < m; i++) z += ys[i] * V[(size_t)i * ld + d];
     x[d] += z;
   }
 }
@@ -249,9 +249,9 @@ cudaError_t launch_reduce(const double* pin, double* out, int do_sqrt, cudaStrea
   reduce_kernel<<<1, kRedThreads, 0, st>>>(pin, out, do_sqrt);
   return cudaGetLastError();
 }
-cudaError_t launch_combine(double* x, const double* V, int n, const double* y, int m, cudaStream_t st) {
+cudaError_t launch_combine(double* x, const double* V, int n, size_t ld, const double* y, int m, cudaStream_t st) {
   if (m > 256) return cudaErrorInvalidValue;
-  combine_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(x, V, n, y, m);
+  combine_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(x, V, n, ld, y, m);
   return cudaGetLastError();
 }
 cudaError_t launch_state_update(double* U, double* U0, const double* du, int n, cudaStream_t st) {
