@@ -27,7 +27,7 @@ void free_all(cfdv_ctx* c) {
   dfree(c->d_x); dfree(c->d_conn); dfree(c->d_bc); dfree(c->d_mask); dfree(c->d_cleng);
   dfree(c->d_csr_ptr); dfree(c->d_csr_idx);
   dfree(c->d_U); dfree(c->d_U0); dfree(c->d_du);
-  dfree(c->d_R64); dfree(c->d_R32); dfree(c->d_rhs); dfree(c->d_s); dfree(c->d_Y64); dfree(c->d_Y32);
+  dfree(c->d_R64); dfree(c->d_R32); dfree(c->d_rhs); dfree(c->d_s); dfree(c->d_prim); dfree(c->d_Y64); dfree(c->d_Y32);
   dfree(c->d_marks);
   dfree(c->d_V); dfree(c->d_W); dfree(c->d_b); dfree(c->d_pa); dfree(c->d_pb); dfree(c->d_H); dfree(c->d_sc);
   dfree(c->d_y); dfree(c->d_rms); dfree(c->d_status); dfree(c->d_pers); dfree(c->d_pers_int); dfree(c->d_Dinv); dfree(c->d_Z);
@@ -212,7 +212,7 @@ int setup_mesh(cfdv_ctx* c, const cfdv_mesh* m) {
       (rc = dalloc(c, &c->d_csr_idx, idx.size())) || (rc = dalloc(c, &c->d_U, (size_t)c->n_dof)) ||
       (rc = dalloc(c, &c->d_U0, (size_t)c->n_dof)) || (rc = dalloc(c, &c->d_du, (size_t)c->n_dof)) ||
       (rc = dalloc(c, &c->d_R64, E * Ke * Ke)) || (rc = dalloc(c, &c->d_rhs, E * Ke)) ||
-      (rc = dalloc(c, &c->d_s, E * 4)) || (rc = dalloc(c, &c->d_Y64, E * Ke)) ||
+      (rc = dalloc(c, &c->d_s, E * 4)) || (rc = dalloc(c, &c->d_prim, (size_t)c->n_nodes * kPrimLd)) || (rc = dalloc(c, &c->d_Y64, E * Ke)) ||
       (rc = dalloc(c, &c->d_Y32, E * Ke)) || (rc = dalloc(c, &c->d_W, (size_t)c->n_dof)) ||
       (rc = dalloc(c, &c->d_b, (size_t)c->n_dof)) || (rc = dalloc(c, &c->d_pa, (size_t)kRedBlocks * 10)) ||
       (rc = dalloc(c, &c->d_pb, (size_t)kRedBlocks * 10)) || (rc = dalloc(c, &c->d_sc, 16)) ||
@@ -939,6 +939,11 @@ int form_enqueue(cfdv_ctx* c, double dt, const double* dt_dev, int precision) {
   gauss_legendre(2, a.gz, a.gw);
   a.n_elements = c->n_elements;
   a.physical_3d_flux = c->phys3d;
+  // node records and FDV parameters by passes of their own above 4096 elements: their two launches
+  // take about 8 us, which the blocks' shorter chains win back from there on (us, own / in the block:
+  // 1024 quads 53.7 / 46.6, 4096 quads 94.8 / 93.7, 20,000 quads 277 / 310; 2275 hexes 95.6 / 93.8,
+  // 5000 hexes 152 / 160, 24,576 hexes 544 / 622)
+  a.prim = c->n_elements > 4096 ? c->d_prim : nullptr;
   a.U = c->d_U; a.x = c->d_x; a.conn = c->d_conn; a.bc = c->d_bc; a.rowmask = c->d_mask;
   a.hnm_idx = c->d_hnm_idx; a.hnm = c->d_hnm;
   a.R64 = c->d_R64;
@@ -950,6 +955,11 @@ int form_enqueue(cfdv_ctx* c, double dt, const double* dt_dev, int precision) {
     cudaEventCreate(&ev.first);
     cudaEventCreate(&ev.second);
     cudaEventRecord(ev.first, c->st);
+  }
+  if (a.prim) {
+    CK(launch_node_records(c->ndim, c->d_U, c->d_x, c->n_nodes, c->d_conn, c->n_elements, c->gas, c->d_prim, c->d_s,
+                           c->st));
+    c->launches += 2;
   }
   CK(launch_form(c->ndim, a, c->st));
   c->launches++;

@@ -76,6 +76,9 @@ inline void gauss_legendre(int N, double* zeta, double* w) {
   }
 }
 
+// A node's record: E, T, U[5], v[3], 1, p, then its Mach and Reynolds numbers
+constexpr int kPrimLd = 14, kPrimMach = 12, kPrimRe = 13;
+
 // Everything the element-formation kernel reads.
 struct FormArgs {
   GasParams gas;
@@ -86,6 +89,7 @@ struct FormArgs {
   int physical_3d_flux;      // 1: evaluate the 3D convective flux the reference drops
   const double* U;           // [Nn][neqn] conserved state
   const double* x;           // [Nn][ndim]
+  const double* prim;        // [Nn][kPrimLd] node records of the state, or null: every block forms its own
   const int* conn;           // [E][nnod]
   const int* bc;             // [E][nface]
   const uint64_t* rowmask;   // [E] Dirichlet rows after ApplyBC
@@ -94,7 +98,7 @@ struct FormArgs {
   double* R64;               // [E][Ke*Ke] column-major per element (FP64 output) or null
   float* R32;                // [E][Ke*Ke] (FP32 output) or null
   double* rhs;               // [E][Ke]
-  double* s_out;             // [E][4] FDV parameters s1..s4 (may be null)
+  double* s_out;             // [E][4] FDV parameters s1..s4: written (may be null), or with prim read
   int* status;               // error flags (non-finite element matrix -> bit 0)
 };
 

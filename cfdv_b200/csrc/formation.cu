@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(FormTraits<3>::THREADS, CFDV_FORM3D_BLOCKS) fd
   int bad = 0;
   hex_load(a, sh, e, tid);
   __syncthreads();
-  hex_geom_jac(sh, tid);
+  hex_geom_jac(a, sh, tid);
   __syncthreads();
   hex_dphi(a, sh, tid);
   __syncthreads();
@@ -62,6 +62,46 @@ __global__ void __launch_bounds__(FormTraits<3>::THREADS, CFDV_FORM3D_BLOCKS) fd
   }
   hex_write(a, sh, e, tid, &bad);
   if (bad) atomicOr(a.status, STATUS_NONFINITE_MATRIX);
+}
+
+// node records of the state U, one thread per node
+template <int NDIM>
+__global__ void __launch_bounds__(128) node_record_kernel(const double* __restrict__ U, const double* __restrict__ x,
+                                                          int n_nodes, GasParams g, double* __restrict__ prim) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= n_nodes) return;
+  double f[kPrimLd];
+  node_record<NDIM>(g, U + (size_t)n * (NDIM + 2), x + (size_t)n * NDIM, f);
+#pragma unroll
+  for (int k = 0; k < kPrimLd; k += 2)
+    *reinterpret_cast<double2*>(prim + (size_t)n * kPrimLd + k) = make_double2(f[k], f[k + 1]);
+}
+
+// s1..s4 of every element from its nodes' Mach and Reynolds numbers, one thread per element and pair
+template <int NNOD>
+__global__ void __launch_bounds__(128) fdv_param_kernel(const double* __restrict__ prim, const int* __restrict__ conn,
+                                                        int E, double* __restrict__ s_out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, e = t >> 1, which = t & 1;
+  if (e >= E) return;
+  double val[NNOD], s[4];
+#pragma unroll
+  for (int i = 0; i < NNOD; i++) val[i] = prim[(size_t)conn[(size_t)e * NNOD + i] * kPrimLd + kPrimMach + which];
+  fdv_pair<NNOD>(val, which, s);
+  *reinterpret_cast<double2*>(s_out + (size_t)e * 4 + 2 * which) =
+      which ? make_double2(s[2], s[3]) : make_double2(s[0], s[1]);
+}
+
+cudaError_t launch_node_records(int ndim, const double* U, const double* x, int n_nodes, const int* conn, int E,
+                                const GasParams& g, double* prim, double* s_out, cudaStream_t st) {
+  const int gn = (n_nodes + 127) / 128, ge = (2 * E + 127) / 128;
+  if (ndim == 2) {
+    node_record_kernel<2><<<gn, 128, 0, st>>>(U, x, n_nodes, g, prim);
+    fdv_param_kernel<4><<<ge, 128, 0, st>>>(prim, conn, E, s_out);
+  } else {
+    node_record_kernel<3><<<gn, 128, 0, st>>>(U, x, n_nodes, g, prim);
+    fdv_param_kernel<8><<<ge, 128, 0, st>>>(prim, conn, E, s_out);
+  }
+  return cudaGetLastError();
 }
 
 cudaError_t launch_form(int ndim, const FormArgs& a, cudaStream_t st) {

@@ -216,6 +216,24 @@ CFDV_HD CFDV_INLINE void node_mach_re(const GasT<S>& g, const NodePrimT<S>& n, S
   *Re = RN_DIV(RN_MUL(n.rho, V), gas_mu(g, Tn));
 }
 
+// A node's record (kPrimLd): unpacked primitives with the node's Mach and Reynolds numbers.  Above a
+// few thousand elements a pass over the nodes forms the records once per formation (FormArgs::prim)
+// and a pass over the elements the FDV parameters: formed in every element's block, a few lanes of
+// one warp spent about 800 instructions of divisions, square roots and powers on them, at the head
+// of the block's chain of barriers.
+template <int NDIM>
+CFDV_HD CFDV_INLINE void node_record(const GasParams& g, const double* U, const double* x, double* f) {
+  NodePrim nd;
+  node_unpack<NDIM>(g, U, x, nd);
+  f[0] = nd.E;
+  f[1] = nd.T;
+  for (int k = 0; k < 5; k++) f[2 + k] = k < NDIM + 2 ? nd.U[k] : 0.0;
+  for (int k = 0; k < 3; k++) f[7 + k] = k < NDIM ? nd.v[k] : 0.0;
+  f[10] = 1.0;
+  f[11] = nd.p;
+  node_mach_re<NDIM>(g, nd, &f[kPrimMach], &f[kPrimRe]);
+}
+
 // FDVParam.h:15-111 over the element's nodes: which = 0 gives s1 and s2 from the Mach
 // numbers, which = 1 gives s3 and s4 from the Reynolds numbers, into s[2*which], s[2*which+1]
 template <int NNOD, class S>
@@ -262,9 +280,24 @@ CFDV_HD CFDV_INLINE void step_load(const FormArgs& a, FormShared<NDIM>& sh, int 
   using T = FormTraits<NDIM>;
   if (tid < T::NNOD) {
     const int n = a.conn[(size_t)e * T::NNOD + tid];
-    node_unpack<NDIM>(a.gas, a.U + (size_t)n * T::NEQ, a.x + (size_t)n * NDIM, sh.nd[tid]);
-    node_mach_re<NDIM>(a.gas, sh.nd[tid], &sh.Mn[tid], &sh.Ren[tid]);
+    NodePrim& nd = sh.nd[tid];
+    double f[kPrimLd];
+    if (a.prim) {
+      for (int k = 0; k < kPrimLd; k++) f[k] = a.prim[(size_t)n * kPrimLd + k];
+    } else {
+      node_record<NDIM>(a.gas, a.U + (size_t)n * T::NEQ, a.x + (size_t)n * NDIM, f);
+      sh.Mn[tid] = f[kPrimMach];
+      sh.Ren[tid] = f[kPrimRe];
+    }
+    nd.E = f[0];
+    nd.T = f[1];
+    for (int k = 0; k < T::NEQ; k++) nd.U[k] = f[2 + k];
+    for (int k = 0; k < NDIM; k++) nd.v[k] = f[7 + k];
+    nd.rho = nd.U[0];
+    nd.p = f[11];
+    for (int k = 0; k < NDIM; k++) nd.x[k] = a.x[(size_t)n * NDIM + k];
   }
+  if (a.prim && tid >= 8 && tid < 12) sh.s[tid - 8] = a.s_out[(size_t)e * 4 + tid - 8];
   if (tid == 32 % T::THREADS) {
     int nf = 0;
     for (int f = 0; f < T::NFACE; f++) {
@@ -306,7 +339,7 @@ CFDV_HD CFDV_INLINE void step_geom_jac(const FormArgs& a, FormShared<NDIM>& sh, 
       plain_jac_2d(z, x4, sl.g.pjac);
     }
   }
-  if (tid >= T::THREADS - 2) {
+  if (!a.prim && tid >= T::THREADS - 2) {
     const int which = tid - (T::THREADS - 2);
     fdv_pair<T::NNOD>(which ? sh.Ren : sh.Mn, which, sh.s);
   }
@@ -964,7 +997,7 @@ CFDV_HD CFDV_INLINE void phase_write(const FormArgs& a, FormShared<NDIM>& sh, in
     if (!(v == v) || v - v != 0.0) *bad = 1;
     a.rhs[(size_t)e * KE + tid] = v;
   }
-  if (tid == 0 && a.s_out)
+  if (!a.prim && tid == 0 && a.s_out)
     for (int i = 0; i < 4; i++) a.s_out[(size_t)e * 4 + i] = sh.s[i];
 }
 

@@ -13,7 +13,9 @@
 // for 256 multiply-adds, where the scalar form took 8 and one shared-memory load per 1.5 of
 // them; the earlier scalar kernel was bound by issue and shared-memory loads (46% of the issue
 // slots, 20% of the FP64 pipe).  Formation of the 128x64x32 ramp (262,144 elements, FP64 and FP32
-// copies): 10.9 -> 5.6 ms; of 2,275 elements 171 -> 94 us.  The result of the G product is, lane by lane, the A operand
+// copies): 10.9 -> 4.7 ms; of 2,275 elements 171 -> 94 us.  By step, of 65,536 elements alone: up
+// to the Jacobian rows 0.49 ms, h 0.14, the contraction 0.30 (its 312 products an element at the
+// matrix rate: 0.29), the store 0.13, boundary faces 0.19.  The result of the G product is, lane by lane, the A operand
 // of the second one: the G tile's columns are ordered (c, r s parity), so no lane moves data.
 //
 // The flux Jacobians are evaluated by row: one thread per (Gauss point, direction i, row r) has
@@ -41,6 +43,20 @@ CFDV_HD CFDV_INLINE void mma_f64(int lane, FA A, FB B, double& c0, double& c1) {
     c0 += A(lane >> 2, k) * B(k, 2 * (lane & 3));
     c1 += A(lane >> 2, k) * B(k, 2 * (lane & 3) + 1);
   }
+#endif
+}
+
+// the product alone: c = A B
+template <class FA, class FB>
+CFDV_HD CFDV_INLINE void mma_f64_fresh(int lane, FA A, FB B, double& c0, double& c1) {
+#ifdef __CUDA_ARCH__
+  const double a = A(lane >> 2, lane & 3), b = B(lane & 3, lane >> 2), z = 0.0;
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %4};"
+      : "=d"(c0), "=d"(c1)
+      : "d"(a), "d"(b), "d"(z));
+#else
+  c0 = c1 = 0.0;
+  mma_f64(lane, A, B, c0, c1);
 #endif
 }
 
@@ -112,7 +128,7 @@ static constexpr HexCTable kHexCTable = make_hex_c_table();
 // ---- block state --------------------------------------------------------------------------
 constexpr int kHexNodeLd = 12;  // node fields E, T, U[5], v[3], 1, p
 constexpr int kHexTileLd = 42;  // column stride of the element-matrix tile (bank-conflict free)
-constexpr int kHexTLd = 300;    // T of a Gauss point: (r s, c, i) at (5 r + s) * 12 + 3 c + i
+constexpr int kHexTLd = 312;    // T of a Gauss point: (r s, c, i) at (5 r + s) * 12 + 3 c + i, and one entry of room
 
 struct HexGp {  // one Gauss point; an odd number of doubles
   GpState st;           // flow state (edited on boundary faces)
@@ -138,7 +154,8 @@ struct FormShared<3> {
   double P[8][16];               // dt Fbar(i, r) - dt^2/2 sum_s A_i(r, s) divF(s) at 5 i + r
   double rhs[40];
   double Mn[8], Ren[8];
-  double s[4], dt, dtsq_2;
+  double s[4], dt, dtsq_2, reinv, rCv;  // reinv = 1 / Re, rCv = 1 / Cv
+  double delta[26 * 4];          // T_c0 of the entries: delta_rs at c = 0
   uint64_t mask;
   int faces[6], codes[6], nfaces, hnm;
   union {
@@ -156,22 +173,26 @@ CFDV_HD CFDV_INLINE HexGp& hex_gp(FormShared<3>& sh, int q) {
 }
 
 // ---- steps ---------------------------------------------------------------------------------
-// load: node unpack, boundary faces, shape functions and natural derivatives (q, N)
+// load: node records, boundary faces, FDV parameters, shape functions and natural derivatives (q, N)
 CFDV_HD CFDV_INLINE void hex_load(const FormArgs& a, FormShared<3>& sh, int e, int tid) {
-  if (tid < 8) {
-    const int n = a.conn[(size_t)e * 8 + tid];
-    NodePrim nd;
-    node_unpack<3>(a.gas, a.U + (size_t)n * 5, a.x + (size_t)n * 3, nd);
-    double* f = sh.F + tid * kHexNodeLd;
-    f[0] = nd.E;
-    f[1] = nd.T;
-    for (int k = 0; k < 5; k++) f[2 + k] = nd.U[k];
-    for (int k = 0; k < 3; k++) f[7 + k] = nd.v[k];
-    f[10] = 1.0;
-    f[11] = nd.p;
-    for (int k = 0; k < 3; k++) sh.x[tid][k] = nd.x[k];
-    node_mach_re<3>(a.gas, nd, &sh.Mn[tid], &sh.Ren[tid]);
-  } else if (tid == 32) {
+  const int* conn = a.conn + (size_t)e * 8;
+  if (a.prim) {
+    if (tid < 96) {
+      sh.F[tid] = a.prim[(size_t)conn[tid / kHexNodeLd] * kPrimLd + tid % kHexNodeLd];
+    } else if (tid < 120) {
+      sh.x[(tid - 96) / 3][tid % 3] = a.x[(size_t)conn[(tid - 96) / 3] * 3 + tid % 3];
+    } else if (tid < 124) {
+      sh.s[tid - 120] = a.s_out[(size_t)e * 4 + tid - 120];
+    }
+  } else if (tid < 8) {
+    double f[kPrimLd];
+    node_record<3>(a.gas, a.U + (size_t)conn[tid] * 5, a.x + (size_t)conn[tid] * 3, f);
+    for (int k = 0; k < kHexNodeLd; k++) sh.F[tid * kHexNodeLd + k] = f[k];
+    for (int k = 0; k < 3; k++) sh.x[tid][k] = a.x[(size_t)conn[tid] * 3 + k];
+    sh.Mn[tid] = f[kPrimMach];
+    sh.Ren[tid] = f[kPrimRe];
+  }
+  if (tid == 124) {
     int nf = 0;
     for (int f = 0; f < 6; f++) {
       const int c = a.bc[(size_t)e * 6 + f];
@@ -186,8 +207,12 @@ CFDV_HD CFDV_INLINE void hex_load(const FormArgs& a, FormShared<3>& sh, int e, i
     sh.mask = a.rowmask ? a.rowmask[e] : 0ull;
     sh.dt = a.dt_dev ? *a.dt_dev : a.dt;
     sh.dtsq_2 = a.dt_dev ? sh.dt * sh.dt / 2.0 : a.dtsq_2;
-  } else if (tid >= 64) {
-    const int q = (tid - 64) >> 3, N = (tid - 64) & 7;
+  }
+  if (tid == 96) sh.reinv = 1.0 / a.gas.creyn;
+  if (tid == 97) sh.rCv = 1.0 / a.gas.Cv;
+  if (tid < 104) sh.delta[tid] = (tid % 4 == 0 && (tid / 4) % 6 == 0) ? 1.0 : 0.0;
+  if (tid < 64) {
+    const int q = tid >> 3, N = tid & 7;
     const int hi = a.hnm_idx ? a.hnm_idx[e] : -1;
     if (hi < 0) {  // shape_fn<3> for one node
       const double zx = a.gz[q >> 2], zy = a.gz[(q >> 1) & 1], zz = a.gz[q & 1];
@@ -212,17 +237,16 @@ CFDV_HD CFDV_INLINE void hex_load(const FormArgs& a, FormShared<3>& sh, int e, i
   }
 }
 
-// isoparametric Jacobian entries (q, i, k); FDV parameters of the element (two threads)
-CFDV_HD CFDV_INLINE void hex_geom_jac(FormShared<3>& sh, int tid) {
+// isoparametric Jacobian entries (q, i, k); without node records, FDV parameters (two threads)
+CFDV_HD CFDV_INLINE void hex_geom_jac(const FormArgs& a, FormShared<3>& sh, int tid) {
   if (tid < 72) {
     const int q = tid / 9, ik = tid % 9, i = ik / 3, k = ik % 3;
     double j = 0.0;
 #pragma unroll
     for (int N = 0; N < 8; N++) j = RN_ADD(j, RN_MUL(sh.cM[q][4 * N + 1 + k], sh.x[N][i]));
     sh.jac[q][ik] = j;
-  } else if (tid >= 126) {
-    fdv_pair<8>(tid == 127 ? sh.Ren : sh.Mn, tid - 126, sh.s);
   }
+  if (!a.prim && tid >= 126) fdv_pair<8>(tid == 127 ? sh.Ren : sh.Mn, tid - 126, sh.s);
 }
 
 // physical derivatives (q, N): every thread of a point inverts the point's Jacobian itself
@@ -344,7 +368,7 @@ template <bool FACE>
 CFDV_HD CFDV_INLINE void hex_rows(const FormArgs& a, FormShared<3>& sh, int tid) {
   constexpr int NQ = FACE ? 4 : 8, NT = 3 * NQ;
   const double dt = sh.dt, h2 = sh.dtsq_2, s1 = sh.s[0], s2 = sh.s[1], s3 = sh.s[2], s4 = sh.s[3];
-  const double reinv = 1.0 / a.gas.creyn;
+  const double reinv = sh.reinv;
   if (tid < 4 * NT) {
     const int r = 1 + tid / NT, q = (tid % NT) / 3, i = tid % 3;
     HexGp& g = hex_gp<FACE>(sh, q);
@@ -368,7 +392,7 @@ CFDV_HD CFDV_INLINE void hex_rows(const FormArgs& a, FormShared<3>& sh, int tid)
       av[4] = d ? g1 : 0.0;
       bv[4] = 0.0;
     } else {
-      const double E = f.E, gE = a.gas.gamma * E, T1 = f.k * irho * irho / a.gas.Cv;
+      const double E = f.E, gE = a.gas.gamma * E, T1 = f.k * irho * irho * sh.rCv;
       double vm = 0.0, mv = 0.0, wt = 0.0;  // v.d_i m, v.grad m_i, w.tau_i
 #pragma unroll
       for (int k = 0; k < 3; k++) {
@@ -409,7 +433,7 @@ CFDV_HD CFDV_INLINE void hex_rows(const FormArgs& a, FormShared<3>& sh, int tid)
     HexGp& g = hex_gp<FACE>(sh, q);
     const GpState& f = g.st;
     const double sc = -dt * s3 * reinv * g.irho;
-    const double M = sc * f.mu, L = -2.0 / 3.0 * M, K = sc * f.k / a.gas.Cv;
+    const double M = sc * f.mu, L = -2.0 / 3.0 * M, K = sc * f.k * sh.rCv;
     const double* w = g.w;
     const double W2 = w[0] * w[0] + w[1] * w[1] + w[2] * w[2];
     double dF = 0.0;
@@ -466,29 +490,43 @@ CFDV_HD CFDV_INLINE void hex_hmat(const FormArgs& a, FormShared<3>& sh, int tid)
 #else
   const unsigned long long slots = kHexCTable.v[lane];
 #endif
+  // this lane's entries: rows 8 mt + lane / 4, columns 8 nt + 2 (lane % 4) + e (of 15 each); the
+  // column's part of T's index and whether row 0 of D_j (s2 at s = 1 + j alone) reaches it
+  int tcol[2][2];
+  double sd[2][2];
+#pragma unroll
+  for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int col = 8 * nt + 2 * (lane & 3) + e, j = col / 5, s = col % 5;
+      tcol[nt][e] = 12 * s + 3 + 3 * j;
+      sd[nt][e] = s == 1 + j ? s2h : 0.0;
+    }
+  const bool last = (lane & 3) == 3;  // column 15 is not one
+#pragma unroll 1
   for (int q = tid >> 5; q < NQ; q += 4) {
     HexGp& g = hex_gp<FACE>(sh, q);
     double* Tq = sh.T[q];
 #pragma unroll
     for (int mt = 0; mt < 2; mt++) {
-      const int row = 8 * mt + (lane >> 2), i = row / 5, r = row % 5;
-      const double a0 = s2h * g.A[row][0];
+      const int row = 8 * mt + (lane >> 2);
+      const int trow = 60 * (row % 5) + row / 5;
+      const double a0 = g.A[row][0];
+      double c[2][2];
 #pragma unroll
       for (int nt = 0; nt < 2; nt++) {
-        double c[2];
 #pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const int col = 8 * nt + 2 * (lane & 3) + e, j = col / 5, s = col % 5;
-          // row 0 of D_j is s2 at s = 1 + j alone
-          c[e] = g.ctab[(slots >> (8 * (4 * mt + 2 * nt + e))) & 31u] + (s == 1 + j ? a0 : 0.0);
-        }
+        for (int e = 0; e < 2; e++)
+          c[nt][e] = g.ctab[(slots >> (8 * (4 * mt + 2 * nt + e))) & 31u] + sd[nt][e] * a0;
         mma_f64(lane, [&](int rw, int k) { return g.A[8 * mt + rw][1 + k]; },
-                [&](int k, int cl) { return g.D[k][8 * nt + cl]; }, c[0], c[1]);
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const int col = 8 * nt + 2 * (lane & 3) + e, j = col / 5, s = col % 5;
-          if (row < 15 && col < 15) Tq[(5 * r + s) * 12 + 3 + 3 * j + i] = c[e];
-        }
+                [&](int k, int cl) { return g.D[k][8 * nt + cl]; }, c[nt][0], c[nt][1]);
+      }
+      if (row < 15) {
+        double* t = Tq + trow;
+        t[tcol[0][0]] = c[0][0];
+        t[tcol[0][1]] = c[0][1];
+        t[tcol[1][0]] = c[1][0];
+        if (!last) t[tcol[1][1]] = c[1][1];
       }
     }
   }
@@ -504,7 +542,7 @@ CFDV_HD CFDV_INLINE void hex_hmat(const FormArgs& a, FormShared<3>& sh, int tid)
     } else if (r > 0) {
       fb = -f.tau[i][r - 1] * g.S[0];
     }
-    fb /= a.gas.creyn;
+    fb *= sh.reinv;
     if (a.physical_3d_flux)
       for (int b = 0; b < 8; b++) fb += sh.cM[q][4 * b] * hex_node_conv(sh, b, i, r);
     double u = 0.0;
@@ -528,52 +566,56 @@ CFDV_HD CFDV_INLINE void hex_contract(FormShared<3>& sh, int tid) {
     acc[p][0] = (FACE && p < nrs) ? sh.Rt[at] : 0.0;
     acc[p][1] = (FACE && p < nrs) ? sh.Rt[at + 5 * kHexTileLd] : 0.0;
   }
+#ifdef __CUDA_ARCH__
+  // the G operand of pair p at this lane: row k of column (c, e): T for k > 0, the delta table for
+  // k = 0, stepping by the pair and by the point (entry 25 is the row of room: its tile is unused)
+  const int kk = lane & 3, c4 = N >> 1, e4 = N & 1;
+  const double* tp = kk ? sh.T[0] + (rs0 + e4) * 12 + 3 * c4 + kk - 1 : sh.delta + (rs0 + e4) * 4 + c4;
+  const int dp = kk ? 24 : 8, dq = kk ? kHexTLd : 0;
+  const double *t0 = tp, *t1 = tp + dp, *t2 = tp + 2 * dp, *t3 = nrs == 8 ? tp + 3 * dp : tp;
+#endif
 #pragma unroll 1
   for (int q = 0; q < NQ; q++) {
     const double* cq = sh.cM[q];
-    const double* Tq = sh.T[q];
     auto A1 = [&](int row, int k) -> double {
       if (FACE) return k == 0 ? 0.0 : -(cq[4 * row] * sh.en[q][k - 1]);
       return sh.wJ[q] * cq[4 * row + k];
     };
     auto B2 = [&](int k, int col) -> double { return cq[4 * col + k]; };
+    auto PB = [&](int k, int col) -> double { return (k > 0 && col < 5) ? sh.P[q][5 * (k - 1) + col] : 0.0; };
 #ifdef __CUDA_ARCH__
-    const double a1 = A1(N, lane & 3), b2 = B2(lane & 3, N);
+    const double b2 = B2(lane & 3, N), a1 = FACE ? A1(N, lane & 3) : sh.wJ[q] * b2;
     auto rd_a = [&](int, int) { return a1; };
     auto rd_b = [&](int, int) { return b2; };
-#else
-    auto rd_a = A1;
-    auto rd_b = B2;
-#endif
+    const double tv[4] = {*t0, *t1, *t2, *t3};
+    t0 += dq;
+    t1 += dq;
+    t2 += dq;
+    t3 += dq;
 #pragma unroll
     for (int p = 0; p < 4; p++) {
       if (2 * p >= nrs) break;
-      // G tile of entries rs, rs + 1: column 2 c + e is coefficient c of entry rs + e
-      auto TB = [&](int k, int col) -> double {
-        const int rs = rs0 + 2 * p + (col & 1), c = col >> 1;
-        return k == 0 ? ((c == 0 && rs % 6 == 0) ? 1.0 : 0.0) : Tq[(rs < 25 ? rs : 24) * 12 + 3 * c + k - 1];
-      };
-#ifdef __CUDA_ARCH__
-      double g[2] = {0.0, 0.0};
-      mma_f64(lane, rd_a, TB, g[0], g[1]);
-#endif
+      double g[2];
+      mma_f64_fresh(lane, rd_a, [&](int, int) { return tv[p]; }, g[0], g[1]);
 #pragma unroll
-      for (int e = 0; e < 2; e++) {
-#ifdef __CUDA_ARCH__
-        auto rd_g = [&](int, int) { return g[e]; };
+      for (int e = 0; e < 2; e++)
+        mma_f64(lane, [&](int, int) { return g[e]; }, rd_b, acc[2 * p + e][0], acc[2 * p + e][1]);
+    }
+    if (w == 3) mma_f64(lane, rd_a, PB, ar[0], ar[1]);
 #else
+    const double* Tq = sh.T[q];
+    for (int p = 0; 2 * p < nrs; p++)
+      for (int e = 0; e < 2; e++) {
+        const int rs = rs0 + 2 * p + e;
         auto rd_g = [&](int row, int c) {
-          double v = 0.0;
-          for (int k = 0; k < 4; k++) v += A1(row, k) * TB(k, 2 * c + e);
+          double v = A1(row, 0) * sh.delta[4 * rs + c];
+          for (int k = 1; k < 4; k++) v += A1(row, k) * (rs < 25 ? Tq[rs * 12 + 3 * c + k - 1] : 0.0);
           return v;
         };
-#endif
-        mma_f64(lane, rd_g, rd_b, acc[2 * p + e][0], acc[2 * p + e][1]);
+        mma_f64(lane, rd_g, B2, acc[2 * p + e][0], acc[2 * p + e][1]);
       }
-    }
-    if (w == 3)
-      mma_f64(lane, rd_a, [&](int k, int col) { return (k > 0 && col < 5) ? sh.P[q][5 * (k - 1) + col] : 0.0; },
-              ar[0], ar[1]);
+    if (w == 3) mma_f64(lane, A1, PB, ar[0], ar[1]);
+#endif
   }
 #pragma unroll
   for (int p = 0; p < 8; p++)
@@ -618,29 +660,35 @@ CFDV_HD CFDV_INLINE void hex_face_geom(const FormArgs& a, FormShared<3>& sh, int
 CFDV_HD CFDV_INLINE void hex_write(const FormArgs& a, FormShared<3>& sh, int e, int tid, int* bad) {
   const uint64_t mk = sh.mask;
   const size_t base = (size_t)e * 1600;
-  bool nf = false;
-  for (int k = tid; k < 800; k += 128) {
-    const int J = k / 20, I = 2 * (k % 20);
-    double v0 = sh.Rt[J * kHexTileLd + I], v1 = sh.Rt[J * kHexTileLd + I + 1];
+  double nf = 0.0;  // v * 0 is NaN for an entry that is not finite, and stays
+  if (tid < 120) {  // rows I, I + 1 of columns tid / 20, + 6, ...: one row pair per thread
+    const int I = 2 * (tid % 20);
     const unsigned m2 = (unsigned)(mk >> I) & 3u;
-    if (m2 & 1u) v0 = I == J ? 0.5 : 0.0;
-    if (m2 & 2u) v1 = I + 1 == J ? 0.5 : 0.0;
-    nf |= (v0 - v0 != 0.0) || (v1 - v1 != 0.0);
+    for (int J = tid / 20; J < 40; J += 6) {
+      const double* t = sh.Rt + J * kHexTileLd + I;
+      double v0 = t[0], v1 = t[1];
+      if (m2) {
+        if (m2 & 1u) v0 = I == J ? 0.5 : 0.0;
+        if (m2 & 2u) v1 = I + 1 == J ? 0.5 : 0.0;
+      }
+      nf += v0 * 0.0 + v1 * 0.0;
+      const size_t at = base + J * 40 + I;
 #ifdef __CUDA_ARCH__
-    if (a.R64) *reinterpret_cast<double2*>(a.R64 + base + 2 * k) = make_double2(v0, v1);
-    if (a.R32) *reinterpret_cast<float2*>(a.R32 + base + 2 * k) = make_float2((float)v0, (float)v1);
+      if (a.R64) *reinterpret_cast<double2*>(a.R64 + at) = make_double2(v0, v1);
+      if (a.R32) *reinterpret_cast<float2*>(a.R32 + at) = make_float2((float)v0, (float)v1);
 #else
-    if (a.R64) { a.R64[base + 2 * k] = v0; a.R64[base + 2 * k + 1] = v1; }
-    if (a.R32) { a.R32[base + 2 * k] = (float)v0; a.R32[base + 2 * k + 1] = (float)v1; }
+      if (a.R64) { a.R64[at] = v0; a.R64[at + 1] = v1; }
+      if (a.R32) { a.R32[at] = (float)v0; a.R32[at + 1] = (float)v1; }
 #endif
+    }
   }
   if (tid < 40) {
     const double v = ((mk >> tid) & 1ull) ? 0.0 : sh.rhs[tid];
-    nf |= v - v != 0.0;
+    nf += v * 0.0;
     a.rhs[(size_t)e * 40 + tid] = v;
   }
-  if (nf) *bad = 1;
-  if (tid < 4 && a.s_out) a.s_out[(size_t)e * 4 + tid] = sh.s[tid];
+  if (nf != 0.0) *bad = 1;
+  if (!a.prim && tid < 4 && a.s_out) a.s_out[(size_t)e * 4 + tid] = sh.s[tid];
 }
 
 constexpr int kHexDomainSteps = 8, kHexFaceSteps = 6;
@@ -650,7 +698,7 @@ CFDV_HD CFDV_INLINE int hex_nsteps(const FormShared<3>& sh) { return kHexDomainS
 CFDV_HD CFDV_INLINE void hex_step(int k, const FormArgs& a, FormShared<3>& sh, int e, int tid, int* bad) {
   switch (k) {
     case 0: hex_load(a, sh, e, tid); return;
-    case 1: hex_geom_jac(sh, tid); return;
+    case 1: hex_geom_jac(a, sh, tid); return;
     case 2: hex_dphi(a, sh, tid); return;
     case 3: hex_state<false>(sh, 0, tid); return;
     case 4: hex_gp_domain(a, sh, tid); return;

@@ -69,6 +69,10 @@ __device__ __forceinline__ double reduce_partials(const double* __restrict__ p, 
 
 // ---- launchers ---------------------------------------------------------------
 struct FormArgs;
+// node records (kPrimLd doubles a node) of the state U and s1..s4 of every element: what the
+// formation reads
+cudaError_t launch_node_records(int ndim, const double* U, const double* x, int n_nodes, const int* conn, int E,
+                                const GasParams& g, double* prim, double* s_out, cudaStream_t st);
 cudaError_t launch_form(int ndim, const FormArgs& a, cudaStream_t st);
 // FDVParam's s1 > threshold per element from the node states U (refinement marks, 1 byte each)
 cudaError_t launch_refine_marks(int ndim, const double* U, const double* x, const int* conn, int E, const GasParams& g,
