@@ -400,7 +400,7 @@ int persistent_args(cfdv_ctx* c, int m, int restarts, int orth, double rtol, Per
   a.rtol = rtol;
   a.conn = c->d_conn; a.csr_ptr = c->d_csr_ptr; a.csr_idx = c->d_csr_idx;
   a.R64 = c->d_R64; a.R32 = c->d_R32; a.Y64 = c->d_Y64; a.Y32 = c->d_Y32;
-  a.b = c->d_b; a.du = c->d_du; a.V = c->d_V; a.ldv = vec_stride(c); a.W = c->d_W;
+  a.b = c->d_b; a.du = c->d_du; a.V = c->d_V; a.ldv = (int)vec_stride(c); a.W = c->d_W;
   a.part0 = c->d_pa; a.part1 = c->d_pb;
   a.H = c->d_H;
   double* p = c->d_pers;

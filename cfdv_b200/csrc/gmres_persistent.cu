@@ -772,7 +772,10 @@ __host__ __device__ constexpr int own_nodes(int n_nodes, int blocks) {
   return NEQ % 2 ? pn + (pn & 1) : pn;
 }
 
-template <int KE, int NEQ, int NNOD, typename TR, bool RES>
+// REF: one cycle of the reference-mode solve (PersistentArgs::ref_cycle).  A kernel of its own: as a
+// run-time branch its estimate made the other solves' critical path longer (resident plate solve,
+// FP64, 0.970 -> 1.020 ms).
+template <int KE, int NEQ, int NNOD, typename TR, bool RES, bool REF>
 __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(PersistentArgs a) {
   extern __shared__ __align__(16) double dyn[];
   const int nb = gridDim.x, tid = threadIdx.x, bid = blockIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -780,7 +783,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
   // own unknowns [lo, lo + ns): whole nodes, S per block
   const int pn = own_nodes<NEQ>(n / NEQ, nb), S = pn * NEQ;
   const int lo = min(n, bid * S), ns = min(n, lo + S) - lo;
-  const size_t ldv = a.ldv;  // stride of the basis vectors (even)
+  const int ldv = a.ldv;  // stride of the basis vectors (even)
   Barrier bar{a.bar_count, a.err, 0u};
   // one tile area for both products (FP64 restart residual, TR Arnoldi products)
   double* tile64 = dyn;
@@ -1114,7 +1117,6 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
   //   slot j+1 = u / sigma (sigma > 0), or u kept in w (sigma = 0); returns the share of ||u||^2
   // pass B by the first nthr threads of the block (the resident path's overlapped step)
   auto pass_b_part = [&](int j, double nu, double pj, double sigma, int nthr) {
-    const Divisor by_nu(nu), by_sigma(sigma);
     for (int dl = tid; dl < ns; dl += nthr) {
       double su = 0.0, sw = 0.0;
 #pragma unroll 4
@@ -1123,23 +1125,14 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
         su += hs1[i] * q;
         sw += hs1[j + i] * q;
       }
-      const double qj = by_nu(vld(j, dl) - su);
+      const double qj = (vld(j, dl) - su) / nu;
       const double u = wld(dl) - sw - pj * qj;
       vst(j, dl, qj);
-      vst(j + 1, dl, by_sigma(u));
+      vst(j + 1, dl, u / sigma);
     }
   };
   auto pass_b = [&](int j, double nu, double pj, double sigma) -> double {
     double acc = 0.0;
-    const Divisor by_nu(nu), by_sigma(sigma > 0.0 ? sigma : 1.0);
-    auto finish = [&](int dl, double u, double w, double su, double sw) {
-      const double qj = by_nu(u - su);
-      const double un = w - sw - pj * qj;
-      vst(j, dl, qj);
-      if (sigma > 0.0) vst(j + 1, dl, by_sigma(un));
-      else wst(dl, un);
-      acc += un * un;
-    };
     if constexpr (!kGs) {
       for (int dl = tid; dl < ns; dl += kThreads) {
         double su = 0.0, sw = 0.0;
@@ -1149,9 +1142,23 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
           su += hs1[i] * q;
           sw += hs1[j + i] * q;
         }
-        finish(dl, vld(j, dl), wld(dl), su, sw);
+        const double qj = (vld(j, dl) - su) / nu;
+        const double u = wld(dl) - sw - pj * qj;
+        vst(j, dl, qj);
+        if (sigma > 0.0) vst(j + 1, dl, u / sigma);
+        else wst(dl, u);
+        acc += u * u;
       }
     } else {
+      const Divisor by_nu(nu), by_sigma(sigma > 0.0 ? sigma : 1.0);
+      auto finish = [&](int dl, double u, double w, double su, double sw) {
+        const double qj = by_nu(u - su);
+        const double un = w - sw - pj * qj;
+        vst(j, dl, qj);
+        if (sigma > 0.0) vst(j + 1, dl, by_sigma(un));
+        else wst(dl, un);
+        acc += un * un;
+      };
       if (gs_k(S) == 1) {
         if (tid == 0) gs_produce<gs_group(1)>(gs, j, true, gs_p, bar);
         if (wid > 0) gs_pass_b<1>(gs, j, W + lo, hs1, hs1 + j, gs_p, bar, finish);
@@ -1226,7 +1233,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
   // by one thread of every block; sets s_stop
   int total_est = 0;
   auto givens = [&](int j, double nrm) {
-    if (tid == kThreads - 1 && a.ref_cycle) {
+    if (REF && tid == kThreads - 1) {
       // the reference's estimate: c, s from the unrotated column (MPI_GMRES.h:696-730)
       const double h = col[j], sn_j = nrm / sqrt(h * h + nrm * nrm);
       g[j + 1] = -sn_j * g[j];
@@ -1261,11 +1268,11 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
 
   int mv = 0, mv64 = 0;
   long passes = 0;  // algorithmic DOF-vector passes of the orthogonalisation and combination
-  bool converged = bnorm == 0.0 && !a.ref_cycle;  // b = 0: du = 0 is the solution
+  bool converged = bnorm == 0.0 && !REF;  // b = 0: du = 0 is the solution
   double beta = 0.0;
   for (int cycle = 0; cycle < a.max_restarts && !converged; cycle++) {
     // r = b - A64 du, beta = ||r||; from du = 0, r = b and beta = ||b||
-    if (cycle == 0 && a.x0_zero) {
+    if (REF && cycle == 0 && a.x0_zero) {
       for (int dl = tid; dl < ns; dl += kThreads) wst(dl, a.b[lo + dl]);
       beta = bnorm;
     } else {
@@ -1284,7 +1291,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
       if (bid == 0 && tid == 0) atomicOr(a.err, 2);
       return;
     }
-    if (beta < atol && !a.ref_cycle) {
+    if (beta < atol && !REF) {
       converged = true;
       break;
     }
@@ -1493,7 +1500,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
       if (!grid_sync(bar)) return;
       if (s_stop) break;
     }
-    if (a.ref_cycle) {  // the host rotates the Hessenberg matrix and substitutes as the reference does
+    if constexpr (REF) {  // the host rotates the Hessenberg matrix and substitutes as the reference does
       if (bid == 0) {
         for (int t = tid; t < k * (m + 1); t += kThreads) a.H[t] = Hf[t];
         if (tid == 0) {
@@ -1572,7 +1579,9 @@ namespace {
 
 template <int KE, int NEQ, int NNOD, typename TR, bool RES>
 cudaError_t launch_cfg(const PersistentArgs& a, int blocks, size_t dyn_bytes, int node_cache, cudaStream_t st) {
-  auto* k = gmres_persistent_kernel<KE, NEQ, NNOD, TR, RES>;
+  auto* k = gmres_persistent_kernel<KE, NEQ, NNOD, TR, RES, false>;
+  if constexpr (sizeof(TR) == 8)
+    if (a.ref_cycle) k = gmres_persistent_kernel<KE, NEQ, NNOD, TR, RES, true>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_bytes);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
@@ -1596,7 +1605,7 @@ cudaError_t launch_one(const PersistentArgs& a, cudaStream_t st) {
   const int pn = own_nodes<NEQ>(a.n_dof / NEQ, blocks), S = pn * NEQ;
   const bool cgs = (a.orth == 0 || a.orth == 2 || a.orth == 3) && a.m + 2 <= kMaxBasis && a.partm != nullptr;
   cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, gmres_persistent_kernel<KE, NEQ, NNOD, TR, true>);
+  cudaError_t e = cudaFuncGetAttributes(&fa, gmres_persistent_kernel<KE, NEQ, NNOD, TR, true, false>);
   if (e != cudaSuccess) return e;
   const size_t res_bytes = sizeof(double) * persistent_dyn_doubles<KE>(a.m, S, true);
   // the node pass's offsets: an entry count and kMaxValence offsets per own node
@@ -1605,7 +1614,7 @@ cudaError_t launch_one(const PersistentArgs& a, cudaStream_t st) {
     return launch_cfg<KE, NEQ, NNOD, TR, true>(a, blocks, res_bytes + cache_bytes, 1, st);
   if (cgs && fa.sharedSizeBytes + res_bytes <= (size_t)optin)
     return launch_cfg<KE, NEQ, NNOD, TR, true>(a, blocks, res_bytes, 0, st);
-  e = cudaFuncGetAttributes(&fa, gmres_persistent_kernel<KE, NEQ, NNOD, TR, false>);
+  e = cudaFuncGetAttributes(&fa, gmres_persistent_kernel<KE, NEQ, NNOD, TR, false, false>);
   if (e != cudaSuccess) return e;
   const bool dcgs = KE == 40 && cgs && a.orth != 0;  // the basis through the ring
   const size_t slot = gs_slot_bytes(S);

@@ -26,7 +26,7 @@ struct PersistentArgs {
   int ref_cycle;               // 1: one Arnoldi cycle of the reference's GMRES: its estimate stops the
                                // cycle, H (unrotated, column-major) and V are the result, du stays
   double* V;                   // (m+1) Krylov vectors, 16-byte aligned
-  size_t ldv;                  // their stride: n_dof rounded up to even
+  int ldv;                     // their stride: n_dof rounded up to even
   double* W;
   const double* Dinv;          // node-block Jacobi inverse (right preconditioning) or null
   double* Z;                   // preconditioned vector z_j = Dinv v_j
