@@ -684,6 +684,9 @@ int cfdv::ctxi::solve_launch(cfdv_ctx* c, const cfdv_gmres_opts* o, const double
   }
   PersistentArgs a;
   if ((rc = persistent_args(c, m, o->restarts, o->orth, o->rtol, &a))) return rc;
+  // with one cycle only, a product with non-finite matrices must still be seen (later cycles start
+  // with one anyway)
+  a.x0_zero = !x0 && o->restarts > 1;
   // A^T: transpose every element block in place (restored after the launch), so the kernel's
   // coalesced row loads stream R_e^T and the block Jacobi inverse is that of A^T
   float* r32 = c->have32 ? c->d_R32 : nullptr;
