@@ -124,6 +124,24 @@ __global__ void cfl_argmin_kernel(const double* __restrict__ U, const int* __res
     }
 }
 
+// the arg-min pair of the CFL kernel above: out = node, element length, the node's U (NEQ entries);
+// node -1 when no pair attains the minimum.  One thread, so that one copy brings them to the host.
+__global__ void cfl_pick_kernel(const int* best, const int* __restrict__ conn, const double* __restrict__ cleng,
+                                const double* __restrict__ U, int nnod, int neqn, double* out) {
+  const int b = *best;
+  const int n = b == 0x7fffffff ? -1 : conn[b];
+  out[0] = (double)n;
+  out[1] = n < 0 ? 0.0 : cleng[b / nnod];
+  for (int k = 0; k < neqn; k++) out[2 + k] = n < 0 ? 0.0 : U[(size_t)n * neqn + k];
+}
+struct NodeAdd {
+  double v[5];
+};
+// y[k] += a.v[k], k < n: one node's unknowns
+__global__ void node_add_kernel(double* y, NodeAdd a, int n) {
+  if ((int)threadIdx.x < n) y[threadIdx.x] += a.v[threadIdx.x];
+}
+
 }  // namespace cfdv
 
 // ---------------------------------------------------------------------------------
@@ -132,16 +150,19 @@ namespace {
 
 constexpr int kThreadsFn = 128;
 
-double host_sum(cfdv_ctx* c, const double* d_v, int n, int* rc) {
-  sum_kernel<<<kRedBlocks, kRedThreads, 0, c->st>>>(d_v, n, c->d_pa);
-  launch_reduce(c->d_pa, c->d_sc + 4, 0, c->st);
-  c->launches += 2;
-  double v = 0.0;
-  cudaError_t e = cudaMemcpyAsync(c->h_pin, c->d_sc + 4, sizeof(double), cudaMemcpyDeviceToHost, c->st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
-  if (e != cudaSuccess) *rc = fail(c, CFDV_ERR_CUDA, std::string("reduction: ") + cudaGetErrorString(e));
-  v = c->h_pin[0];
-  return v;
+// the sums of v[0..n) and, when given, of v2[0..n), with one wait for both
+int host_sums(cfdv_ctx* c, const double* d_v, const double* d_v2, int n, double* s1, double* s2) {
+  const double* v[2] = {d_v, d_v2};
+  for (int k = 0; k < (d_v2 ? 2 : 1); k++) {
+    sum_kernel<<<kRedBlocks, kRedThreads, 0, c->st>>>(v[k], n, c->d_pa);
+    CK(launch_reduce(c->d_pa, c->d_sc + 4 + k, 0, c->st));
+    c->launches += 2;
+  }
+  CK(cudaMemcpyAsync(c->h_pin, c->d_sc + 4, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  CK(cudaStreamSynchronize(c->st));
+  *s1 = c->h_pin[0];
+  if (d_v2) *s2 = c->h_pin[1];
+  return CFDV_OK;
 }
 
 EbeArgs ebe_of(cfdv_ctx* c) {
@@ -191,11 +212,7 @@ int vjp_device(cfdv_ctx* c, double dt, const double* d_w, const double* d_du, do
   c->launches++;
   CK(launch_compose_rhs(ebe_of(c), a.out, d_g, c->d_pa, c->st));
   c->launches++;
-  rc = CFDV_OK;
-  *g_dt = host_sum(c, a.out_dt, (int)E, &rc);
-  if (rc) return rc;
-  *g_mach = host_sum(c, a.out_mach, (int)E, &rc);
-  return rc;
+  return host_sums(c, a.out_dt, a.out_mach, (int)E, g_dt, g_mach);
 }
 
 // dr = (dr/dU) tU + (dr/ddt) t_dt + (dr/dMach) t_mach as a node vector
@@ -265,12 +282,7 @@ int wall_force_device(cfdv_ctx* c, int wall_bc, double* F, double* d_gradU, doub
   else force_kernel<3><<<grid, kThreadsFn, 0, c->st>>>(a);
   c->launches++;
   CK(cudaGetLastError());
-  *F = host_sum(c, a.out_val, nl, &rc);
-  if (rc) return rc;
-  if (dF_dmach) {
-    *dF_dmach = host_sum(c, a.out_mach, nl, &rc);
-    if (rc) return rc;
-  }
+  if ((rc = host_sums(c, a.out_val, dF_dmach ? a.out_mach : nullptr, nl, F, dF_dmach))) return rc;
   if (d_gradU) {
     double* eb = c->d_adj_e;  // element-major rows, zero outside the wall elements
     CK(cudaMemsetAsync(eb, 0, sizeof(double) * c->n_elements * Ke, c->st));
@@ -294,20 +306,18 @@ int cfl_sensitivity(cfdv_ctx* c, double cfl, double dt, int* node, double* ddt_d
     cfl_argmin_kernel<3><<<kRedBlocks, 256, 0, c->st>>>(c->d_U, c->d_conn, c->d_cleng, c->n_elements, c->gas, target,
                                                        d_best);
   c->launches++;
-  int best = big;
-  CK(cudaMemcpyAsync(&best, d_best, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+  double* d_pick = c->d_sc + 9;  // node, length, U[5]
+  cfl_pick_kernel<<<1, 1, 0, c->st>>>(d_best, c->d_conn, c->d_cleng, c->d_U, c->nnod, c->neqn, d_pick);
+  c->launches++;
+  CK(cudaMemcpyAsync(c->h_pin, d_pick, 7 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
-  *node = -1;
+  *node = (int)c->h_pin[0];
   for (int k = 0; k < c->neqn; k++) ddt_dU[k] = 0.0;
   *ddt_dmach = 0.0;
-  if (best == big) return CFDV_OK;  // (dt / cfl is attained: cannot happen for a finite dt)
-  const int e = best / c->nnod, i = best % c->nnod;
-  int n = 0;
-  double cl = 0.0, u[5];
-  CK(cudaMemcpy(&n, c->d_conn + (size_t)e * c->nnod + i, sizeof(int), cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(&cl, c->d_cleng + e, sizeof(double), cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(u, c->d_U + (size_t)n * c->neqn, sizeof(double) * c->neqn, cudaMemcpyDeviceToHost));
-  *node = n;
+  if (*node < 0) return CFDV_OK;  // (dt / cfl is attained: cannot happen for a finite dt)
+  const double cl = c->h_pin[1];
+  double u[5];
+  for (int k = 0; k < c->neqn; k++) u[k] = c->h_pin[2 + k];
   for (int dir = 0; dir <= c->neqn; dir++) {
     const GasT<Dual> g = dual_gas(c->gas, dir == c->neqn ? 1.0 : 0.0);
     Dual ud[5], dxn;
@@ -346,12 +356,16 @@ int reload_initial_state(cfdv_ctx* c) {
   return cfdv_load_node_records(c, c->h_records.data(), (size_t)c->n_nodes);
 }
 
-// wall nodes: nodes of faces with the wall code, ascending
-std::vector<int> wall_node_ids(cfdv_ctx* c, int wall_bc, int* rc) {
+// wall nodes: nodes of faces with the wall code, ascending (kept with the mesh for the last code)
+const std::vector<int>& wall_node_ids(cfdv_ctx* c, int wall_bc, int* rc) {
+  std::vector<int>& ids = c->wall_ids;
+  *rc = CFDV_OK;
+  if (c->wall_ids_bc == wall_bc) return ids;
+  ids.clear();
+  c->wall_ids_bc = -1 << 30;
   std::vector<int> bc((size_t)c->n_elements * c->nface), conn((size_t)c->n_elements * c->nnod);
   cudaError_t e1 = cudaMemcpy(bc.data(), c->d_bc, sizeof(int) * bc.size(), cudaMemcpyDeviceToHost);
   cudaError_t e2 = cudaMemcpy(conn.data(), c->d_conn, sizeof(int) * conn.size(), cudaMemcpyDeviceToHost);
-  std::vector<int> ids;
   if (e1 != cudaSuccess || e2 != cudaSuccess) {
     *rc = fail(c, CFDV_ERR_CUDA, "wall nodes: copy of the mesh failed");
     return ids;
@@ -363,7 +377,7 @@ std::vector<int> wall_node_ids(cfdv_ctx* c, int wall_bc, int* rc) {
         for (int i = 0; i < c->nbnod; i++) on[conn[(size_t)e * c->nnod + face_node(c->ndim, f, i)]] = 1;
   for (int n = 0; n < c->n_nodes; n++)
     if (on[n]) ids.push_back(n);
-  *rc = CFDV_OK;
+  c->wall_ids_bc = wall_bc;
   return ids;
 }
 
@@ -461,7 +475,7 @@ int cfdv_wall_nodes(cfdv_ctx* c, int wall_bc, int* ids, int capacity, int* n) {
   if (!c || !n) return CFDV_ERR_ARG;
   cudaSetDevice(c->dev);
   int rc;
-  const std::vector<int> w = wall_node_ids(c, wall_bc, &rc);
+  const std::vector<int>& w = wall_node_ids(c, wall_bc, &rc);
   if (rc) return rc;
   *n = (int)w.size();
   if (ids)
@@ -476,7 +490,7 @@ int cfdv_tangent(cfdv_ctx* c, const cfdv_adjoint_opts* o, double dmach, const do
   if (rc) return rc;
   cudaSetDevice(c->dev);
   if ((rc = ensure_adjoint_buffers(c))) return rc;
-  const std::vector<int> wall = wall_node_ids(c, o->wall_bc, &rc);
+  const std::vector<int>& wall = wall_node_ids(c, o->wall_bc, &rc);
   if (rc) return rc;
   const size_t n = c->n_dof;
   double* tU = c->d_adj_v;           // tangent of U
@@ -544,6 +558,13 @@ static int grow_matrix_pool(cfdv_ctx* c, int want, bool mixed) {
   if (!mixed)
     for (auto& p : c->adj_pool32) dfree(p);
   if (!mixed) c->adj_pool32.clear();
+  // a pool that already holds the sets needs no look at the free memory (a call that can take
+  // milliseconds, and took most of a small run's spread)
+  if ((int)c->adj_pool64.size() >= want) {
+    bool full = true;
+    for (int i = 0; i < want && mixed; i++) full = full && i < (int)c->adj_pool32.size() && c->adj_pool32[i];
+    if (full) return want;
+  }
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
   const size_t reserve = std::max((size_t)2 << 30, total_b / 20);
@@ -583,7 +604,7 @@ int cfdv_adjoint(cfdv_ctx* c, const cfdv_adjoint_opts* o, cfdv_adjoint_result* r
   if (rc) return rc;
   cudaSetDevice(c->dev);
   if ((rc = ensure_adjoint_buffers(c))) return rc;
-  const std::vector<int> wall = wall_node_ids(c, o->wall_bc, &rc);
+  const std::vector<int>& wall = wall_node_ids(c, o->wall_bc, &rc);
   if (rc) return rc;
   const size_t n = c->n_dof;
   const int N = o->n_steps, k = o->checkpoint_every;
@@ -726,10 +747,10 @@ int cfdv_adjoint(cfdv_ctx* c, const cfdv_adjoint_opts* o, cfdv_adjoint_result* r
       double ddU[5], ddM;
       if ((rc = cfl_sensitivity(c, o->cfl, dt, &node, ddU, &ddM))) return rc;
       if (node >= 0) {
-        double h[5];
-        CK(cudaMemcpy(h, lam + (size_t)node * c->neqn, sizeof(double) * c->neqn, cudaMemcpyDeviceToHost));
-        for (int q = 0; q < c->neqn; q++) h[q] += g_dt * ddU[q];
-        CK(cudaMemcpy(lam + (size_t)node * c->neqn, h, sizeof(double) * c->neqn, cudaMemcpyHostToDevice));
+        NodeAdd add;
+        for (int q = 0; q < c->neqn; q++) add.v[q] = g_dt * ddU[q];
+        node_add_kernel<<<1, 32, 0, c->st>>>(lam + (size_t)node * c->neqn, add, c->neqn);
+        c->launches++;
       }
       gM += g_m + g_dt * ddM;
       if (step >= 1) {  // J averages F over U_1 .. U_N

@@ -41,6 +41,8 @@ void free_all(cfdv_ctx* c) {
   c->adj_pool32.clear();
   c->n_wall_elems = 0;
   c->wall_bc_cached = -1 << 30;
+  c->wall_ids.clear();
+  c->wall_ids_bc = -1 << 30;
   c->pers_cap = 0;
   if (c->h_pin) cudaFreeHost(c->h_pin);
   c->h_pin = nullptr;

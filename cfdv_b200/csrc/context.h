@@ -81,6 +81,8 @@ struct cfdv_ctx {
   int* d_wall_elems = nullptr;     // elements with a face of the wall code
   double* d_wall_buf = nullptr;
   int n_wall_elems = 0, wall_bc_cached = -1 << 30;
+  std::vector<int> wall_ids;       // wall nodes of code wall_ids_bc
+  int wall_ids_bc = -1 << 30;
   // profiling
   bool prof = false;
   std::vector<cudaEvent_t> ev_pool;
