@@ -1,8 +1,10 @@
 // CUDA kernels for the per-step FDV set-up: element formation (+ ApplyBC) and the
 // CFL time step.  Formation is one thread block per element running the phases of
-// formation.cuh (quad4) or formation_hex.cuh (hex8); the CFL step is a per-element minimum with a deterministic
+// formation.cuh (quad4) or formation_hex.cuh (hex8); the CFL step is a minimum over the element nodes with a deterministic
 // two-level reduction.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "formation.cuh"
 #include "kernels.h"
@@ -148,14 +150,12 @@ __global__ void cfl_partial_kernel(const double* __restrict__ U, const int* __re
                                    unsigned int* count, double cfl, double* dt_out) {
   constexpr int NNOD = (NDIM == 2) ? 4 : 8, NEQ = NDIM + 2;
   double best = 1000.0;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < E; e += gridDim.x * blockDim.x) {
-    double dxele = 1000.0;
-    for (int i = 0; i < NNOD; i++) {
-      const double* u = U + (size_t)conn[(size_t)e * NNOD + i] * NEQ;
-      double dxn;
-      if (cfl_node_len<NDIM>(u, cleng[e], g, &dxn) && dxn < dxele) dxele = dxn;
-    }
-    best = fmin(best, dxele);
+  // one thread per (element, node): a thread per element ran its nodes' divisions and square roots
+  // one after another (2275 hexes 17 -> 7 us)
+  const size_t n = (size_t)E * NNOD;
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
+    double dxn;
+    if (cfl_node_len<NDIM>(U + (size_t)conn[t] * NEQ, cleng[t / NNOD], g, &dxn) && dxn < best) best = dxn;
   }
   best = block_reduce_min(best);
   // the last block to finish takes the min over the block partials: dt = cfl * min (dt stays
@@ -181,6 +181,7 @@ __global__ void cfl_partial_kernel(const double* __restrict__ U, const int* __re
 
 cudaError_t launch_cfl(int ndim, const double* U, const int* conn, const double* cleng, int E, const GasParams& g,
                        double cfl, double* partial, unsigned int* count, int nb, double* dt_out, cudaStream_t st) {
+  nb = (int)std::max<size_t>(1, std::min<size_t>(nb, ((size_t)E * (ndim == 2 ? 4 : 8) + 255) / 256));  // a block without elements only lengthens the last one's wait
   if (ndim == 2) cfl_partial_kernel<2><<<nb, 256, 0, st>>>(U, conn, cleng, E, g, partial, count, cfl, dt_out);
   else cfl_partial_kernel<3><<<nb, 256, 0, st>>>(U, conn, cleng, E, g, partial, count, cfl, dt_out);
   return cudaGetLastError();

@@ -414,8 +414,9 @@ __global__ void combine_precond_kernel(double* du, const double* __restrict__ V,
 
 cudaError_t launch_block_jacobi(int ndim, const int* ptr, const int* idx, const double* R, int n_nodes, double* Dinv,
                                 int* status, const double* rhs, double* b, cudaStream_t st) {
-  if (ndim == 2) block_jacobi_kernel<4, 4><<<kRedBlocks, 128, 0, st>>>(ptr, idx, R, n_nodes, Dinv, status, rhs, b);
-  else block_jacobi_kernel<5, 8><<<kRedBlocks, 128, 0, st>>>(ptr, idx, R, n_nodes, Dinv, status, rhs, b);
+  const int grid = (n_nodes + 31) / 32;  // one warp a block: a small mesh still covers the chip
+  if (ndim == 2) block_jacobi_kernel<4, 4><<<grid, 32, 0, st>>>(ptr, idx, R, n_nodes, Dinv, status, rhs, b);
+  else block_jacobi_kernel<5, 8><<<grid, 32, 0, st>>>(ptr, idx, R, n_nodes, Dinv, status, rhs, b);
   return cudaGetLastError();
 }
 
