@@ -403,9 +403,10 @@ struct GsPos {
     slot = t % r.slots;
   }
 };
+// a slot's value; ordered (memory clobber): it must have been used before the slot is handed back
 __device__ __forceinline__ double lds_f64(unsigned addr) {
   double v;
-  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(addr));
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
   return v;
 }
 
@@ -414,6 +415,9 @@ template <int G>
 __device__ __forceinline__ void gs_produce(const GsRing& r, int j, bool down, GsPos p, const Barrier& bar) {
   unsigned long long policy;
   asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
+  // the vectors were written by the block's threads (generic proxy; they fenced and met since): the
+  // copies below (async proxy) come after
+  asm volatile("fence.proxy.async;" ::: "memory");
   const int nch = r.chunks();
   const GsPos first = p;
   int issued = 0;
@@ -492,14 +496,15 @@ __device__ __forceinline__ void gs_dots(const GsRing& r, int j, const double* w,
       double q[T], s0 = 0.0, s1 = 0.0;
 #pragma unroll
       for (int t = 0; t < T; t++) q[t] = lds_f64(b + ad[t]);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(r.empty + 8u * p.slot);
-      p.next(r);
 #pragma unroll
       for (int t = 0; t < T; t++)
         asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                      : "+d"(s0), "+d"(s1)
-                     : "d"(q[t]), "d"(x[t]));
+                     : "d"(q[t]), "d"(x[t])
+                     : "memory");
+      __syncwarp();  // the slot's values are in use, not only requested, when it is given back
+      if (lane == 0) mbar_arrive(r.empty + 8u * p.slot);
+      p.next(r);
       if constexpr (G == 2) {
         s0 += __shfl_xor_sync(0xffffffffu, s0, 9);
         s1 += __shfl_xor_sync(0xffffffffu, s1, 9);
@@ -580,9 +585,6 @@ __device__ __forceinline__ void gs_pass_b(const GsRing& r, int j, const double* 
       for (int q = 0; q < G; q++)
 #pragma unroll
         for (int k = 0; k < K; k++) v[q][k] = i0 + q < j ? lds_f64(b + (unsigned)(q * r.C) * 8u + x[k]) : 0.0;
-      __syncwarp();
-      if ((threadIdx.x & 31) == 0) mbar_arrive(r.empty + 8u * p.slot);
-      p.next(r);
 #pragma unroll
       for (int q = 0; q < G; q++)
         if (i0 + q < j) {
@@ -593,6 +595,9 @@ __device__ __forceinline__ void gs_pass_b(const GsRing& r, int j, const double* 
             sw[k] += hw * v[q][k];
           }
         }
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) mbar_arrive(r.empty + 8u * p.slot);
+      p.next(r);
     }
 #pragma unroll
     for (int k = 0; k < K; k++)
@@ -1167,7 +1172,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
         if (wid > 0) gs_pass_b<2>(gs, j, W + lo, hs1, hs1 + j, gs_p, bar, finish);
       }
       gs_advance(j);
-      asm volatile("fence.proxy.async.global;" ::: "memory");  // the new slots, before bulk copies read them
+      asm volatile("fence.proxy.async;" ::: "memory");  // the new slots, before bulk copies read them
     }
     return acc;
   };
@@ -1298,7 +1303,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
       break;
     }
     for (int dl = tid; dl < ns; dl += kThreads) vst(0, dl, wld(dl) / beta);
-    if constexpr (kGs) asm volatile("fence.proxy.async.global;" ::: "memory");
+    if constexpr (kGs) asm volatile("fence.proxy.async;" ::: "memory");
     if (a.Dinv) precond_slice(0);
     for (int i = tid; i <= m; i += kThreads) g[i] = i == 0 ? beta : 0.0;
     if (!grid_sync(bar)) return;
@@ -1397,7 +1402,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
           sigma = sqrt(sum_partials(a.part0, nb));
           if (sigma > 0.0)
             for (int dl = tid; dl < ns; dl += kThreads) vst(j + 1, dl, wld(dl) / sigma);
-          if constexpr (kGs) asm volatile("fence.proxy.async.global;" ::: "memory");
+          if constexpr (kGs) asm volatile("fence.proxy.async;" ::: "memory");
         }
         passes += j + 2;
         if (!(sigma > 0.0)) {  // invariant subspace (or a non-finite norm): column j is final
