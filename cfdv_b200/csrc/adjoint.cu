@@ -45,7 +45,8 @@ __global__ void __launch_bounds__(32 * kVjpWarps, 1) vjp_warp_kernel(FunctionalA
 template <int NDIM>
 cudaError_t launch_vjp_warp(const FunctionalArgs& a, cudaStream_t st) {
   const size_t smem = sizeof(WarpVjpShared<NDIM>) * kVjpWarps;
-  static const cudaError_t attr =
+  // at every launch: the limit belongs to the current device's context
+  const cudaError_t attr =
       cudaFuncSetAttribute(vjp_warp_kernel<NDIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (attr != cudaSuccess) return attr;
   const int per_block = WarpVjp<NDIM>::EPW * kVjpWarps;
@@ -69,7 +70,8 @@ __global__ void __launch_bounds__(32 * kJvpWarps) jvp_warp_kernel(FunctionalArgs
 template <int NDIM>
 cudaError_t launch_jvp_warp(const FunctionalArgs& a, cudaStream_t st) {
   const size_t smem = sizeof(WarpJvpShared<NDIM>) * kJvpWarps;
-  static const cudaError_t attr =
+  // at every launch: the limit belongs to the current device's context
+  const cudaError_t attr =
       cudaFuncSetAttribute(jvp_warp_kernel<NDIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (attr != cudaSuccess) return attr;
   const int per_block = WarpJvp<NDIM>::EPW * kJvpWarps;
