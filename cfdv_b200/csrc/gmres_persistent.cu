@@ -43,6 +43,7 @@
 
 #include <algorithm>
 
+#include "bounded_wait.h"
 #include "gmres_persistent.h"
 #include "kernels.h"
 
@@ -56,7 +57,6 @@ constexpr int kMaxBasis = 64;         // CGS2 / DCGS2: m + 2 <= kMaxBasis
 constexpr int kMaxValence = 8;        // node-pass offsets cached for nodes with at most 8 entries
 constexpr int kSlots = 128;           // partial slots of one reduction (DCGS2: 2j + 3)
 constexpr int kPartLd = kRedBlocks;   // partm[i * kPartLd + block]
-constexpr unsigned long long kWaitNs = 2000000000ull;  // 2 s: far above any barrier wait
 constexpr double kPythMin = 1e-4;     // ||w2||^2 / ||w1||^2 below this: recompute the norm
 
 __device__ __forceinline__ unsigned long long now_ns() {
@@ -211,27 +211,35 @@ __device__ __forceinline__ bool mbar_test(unsigned bar, unsigned parity) {
       : "memory");
   return done != 0;
 }
-// wait for the phase of `parity` to complete, at most kWaitNs, and give up early when another
-// block has set the launch's failure bit; false: the launch is failing (bit set here if not yet)
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, const Barrier& b) {
-  if (mbar_test(bar, parity)) return true;
-  const unsigned long long t0 = now_ns();
-  for (unsigned polls = 1;; polls++) {
-    if (mbar_test(bar, parity)) return true;
-    if ((polls & 63u) == 0) {
-      unsigned cnt;
-      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(cnt) : "l"(b.count) : "memory");
-      if (cnt & 0x80000000u) return false;
-      if (now_ns() - t0 > kWaitNs) {
-        atomicOr(b.count, 0x80000000u);
-        atomicOr(b.err, 1);
-        return false;
-      }
-    }
+// a wait for the phase of `parity` of an mbarrier (bounded_wait.h); failing: bit 31 of the grid
+// barrier's count, which another block may have set
+struct MbarWait {
+  unsigned bar, parity;
+  const Barrier& b;
+  __device__ __forceinline__ bool done() const { return mbar_test(bar, parity); }
+  __device__ __forceinline__ unsigned long long now() const { return now_ns(); }
+  __device__ __forceinline__ bool failing() const {
+    unsigned cnt;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(cnt) : "l"(b.count) : "memory");
+    return (cnt & 0x80000000u) != 0;
   }
+  __device__ __forceinline__ void fail() const {
+    atomicOr(b.count, 0x80000000u);
+    atomicOr(b.err, 1);
+  }
+  __device__ __forceinline__ bool all(bool p) const { return __all_sync(0xffffffffu, p) != 0; }
+};
+__device__ __forceinline__ bool mbar_wait_thread(unsigned bar, unsigned parity, const Barrier& b) {
+  MbarWait w{bar, parity, b};
+  return wait_thread(w);
 }
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, const Barrier& b) {
-  return mbar_wait(smem_addr(bar), parity, b);
+__device__ __forceinline__ bool mbar_wait_warp(unsigned bar, unsigned parity, const Barrier& b) {
+  MbarWait w{bar, parity, b};
+  return wait_warp(w);
+}
+__device__ __forceinline__ void mbar_wait_landed(unsigned bar, unsigned parity, const Barrier& b) {
+  MbarWait w{bar, parity, b};
+  wait_landed(w);
 }
 __device__ __forceinline__ void bulk_to_shared(unsigned dst, const void* src, unsigned bytes, unsigned bar,
                                                unsigned long long policy) {
@@ -297,7 +305,7 @@ __device__ __noinline__ void elem_pass_ring(const TM* __restrict__ R, const int*
       int issued = 0;
       for (int t = 0; t < T; t++) {
         const unsigned tt = ring_t + t, sl = tt % kRingStages, k = tt / kRingStages;
-        if (k >= 1 && !mbar_wait(rv.empty + sl, (k - 1) & 1u, bar)) break;
+        if (k >= 1 && !mbar_wait_thread(smem_addr(rv.empty + sl), (k - 1) & 1u, bar)) break;
         const int es = e0 + t * SE, ne = min(SE, e1 - es);
         const unsigned bytes = (unsigned)ne * EB;
         mbar_expect_tx(rv.full + sl, bytes);
@@ -305,11 +313,11 @@ __device__ __noinline__ void elem_pass_ring(const TM* __restrict__ R, const int*
                        smem_addr(rv.full + sl), policy);
         issued = t + 1;
       }
-      // copies still in flight land before the pass ends (the consumers wait for them too;
-      // this covers a pass that is being abandoned)
+      // copies still in flight land before the pass ends, in a failing launch as well (the consumers
+      // wait for them too; this covers a pass that is being abandoned)
       for (int t = max(0, issued - kRingStages); t < issued; t++) {
         const unsigned tt = ring_t + t;
-        mbar_wait(rv.full + tt % kRingStages, (tt / kRingStages) & 1u, bar);
+        mbar_wait_landed(smem_addr(rv.full + tt % kRingStages), (tt / kRingStages) & 1u, bar);
       }
     }
   } else {
@@ -331,7 +339,7 @@ __device__ __noinline__ void elem_pass_ring(const TM* __restrict__ R, const int*
         if (lane + 32 < KE) xw[lane + 32] = xb;
         __syncwarp();
         if (first) {
-          if (!mbar_wait(rv.full + sl, k & 1u, bar)) return;
+          if (!mbar_wait_warp(smem_addr(rv.full + sl), k & 1u, bar)) return;
           first = false;
         }
         const TM* Rs = reinterpret_cast<const TM*>(rv.buf + (size_t)sl * stage_bytes) + (size_t)le * KE * KE;
@@ -346,7 +354,7 @@ __device__ __noinline__ void elem_pass_ring(const TM* __restrict__ R, const int*
         if (lane + 32 < KE) Y[(size_t)e * KE + lane + 32] = acc1;
         __syncwarp();  // xw is rewritten for the next element
       }
-      if (first && !mbar_wait(rv.full + sl, k & 1u, bar)) return;  // no element of this stage: keep phases in step
+      if (first && !mbar_wait_warp(smem_addr(rv.full + sl), k & 1u, bar)) return;  // no element of this stage: keep phases in step
       __syncwarp();
       if (lane == 0) mbar_arrive(rv.empty + sl);
     }
@@ -427,7 +435,7 @@ __device__ __forceinline__ void gs_produce(const GsRing& r, int j, bool down, Gs
     const unsigned bytes = (unsigned)(n + (n & 1)) * 8u;  // an odd tail: the vectors' stride has room for one more
     const double* src = r.V + (size_t)c * r.C;
     for (int i = 0; i < j; i += G) {
-      if (p.fill >= 1 && !mbar_wait(r.empty + 8u * p.slot, (p.fill - 1) & 1u, bar)) { ok = false; break; }
+      if (p.fill >= 1 && !mbar_wait_thread(r.empty + 8u * p.slot, (p.fill - 1) & 1u, bar)) { ok = false; break; }
       const int nv = min(G, j - i);
       mbar_expect_tx(r.full + 8u * p.slot, (unsigned)nv * bytes);
       for (int v = 0; v < nv; v++)
@@ -437,11 +445,11 @@ __device__ __forceinline__ void gs_produce(const GsRing& r, int j, bool down, Gs
       issued++;
     }
   }
-  // copies still in flight land before the pass ends
+  // copies still in flight land before the pass ends, in a failing launch as well
   const int last = min(issued, (int)r.slots);
   p = first;
   p.advance(r, (unsigned)(issued - last));
-  for (int q = 0; q < last; q++, p.next(r)) mbar_wait(r.full + 8u * p.slot, p.fill & 1u, bar);
+  for (int q = 0; q < last; q++, p.next(r)) mbar_wait_landed(r.full + 8u * p.slot, p.fill & 1u, bar);
 }
 
 // Consumer side of the dots: redw[i] = <q_i, u> and, with w, redw[j + i] = <q_i, w> over the
@@ -491,7 +499,7 @@ __device__ __forceinline__ void gs_dots(const GsRing& r, int j, const double* w,
     }
     fetch(c + 1);
     for (int i0 = 0; i0 < j; i0 += G) {
-      if (!mbar_wait(r.full + 8u * p.slot, p.fill & 1u, bar)) return;
+      if (!mbar_wait_warp(r.full + 8u * p.slot, p.fill & 1u, bar)) return;
       const unsigned b = r.buf + p.slot * r.slot_bytes;
       double q[T], s0 = 0.0, s1 = 0.0;
 #pragma unroll
@@ -578,7 +586,7 @@ __device__ __forceinline__ void gs_pass_b(const GsRing& r, int j, const double* 
     }
     fetch(c - 1);
     for (int i0 = 0; i0 < j; i0 += G) {
-      if (!mbar_wait(r.full + 8u * p.slot, p.fill & 1u, bar)) return;
+      if (!mbar_wait_warp(r.full + 8u * p.slot, p.fill & 1u, bar)) return;
       const unsigned b = r.buf + p.slot * r.slot_bytes;
       double v[G][K];
 #pragma unroll
