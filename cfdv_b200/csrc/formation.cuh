@@ -697,11 +697,12 @@ CFDV_HD CFDV_INLINE void edit_face_state_3d(int code, GpStateT<S>& f, const doub
       viscous_stress<3>(f);
       for (int i = 0; i < 3; i++) f.tau[i][0] = 0;
       break;
-    case 7:  // falls through into 77/32 in the reference (eval2dboundary.h:113-145)
+    case 7:  // falls through into 77/32 in the reference (eval2dboundary.h:113-145), which forms the
+             // stress once more: the tau[i][2] that the case had set to zero come back
       f.dT[2] = 0.0;
       f.dT[1] = 0.0;
       viscous_stress<3>(f);
-      for (int i = 0; i < 3; i++) { f.tau[i][2] = 0; f.tau[i][1] = 0; }
+      for (int i = 0; i < 3; i++) f.tau[i][1] = 0;
       break;
     case 77:
     case 32:
