@@ -44,6 +44,7 @@
 #include <algorithm>
 
 #include "bounded_wait.h"
+#include "divisor.h"
 #include "gmres_persistent.h"
 #include "kernels.h"
 
@@ -539,21 +540,6 @@ __device__ __forceinline__ void gs_dots(const GsRing& r, int j, const double* w,
     }
   }
 }
-
-// x / d with the reciprocal of d at hand: one Newton correction of the quotient (Markstein's
-// final step) gives the correctly rounded quotient but for rare last-bit cases, in 3 operations;
-// the compiled division takes about 35 instructions, 3 to 8 us a pass B of 1.38M unknowns.
-// rd not a normal number (d tiny or huge): the division itself.
-struct Divisor {
-  double d, rd;
-  bool fast;
-  __device__ __forceinline__ explicit Divisor(double v) : d(v), rd(1.0 / v), fast(fabs(rd) >= 1e-290 && fabs(rd) <= 1e290) {}
-  __device__ __forceinline__ double operator()(double x) const {
-    if (!fast) return x / d;
-    const double q = x * rd;
-    return fma(fma(-q, d, x), rd, q);
-  }
-};
 
 // Consumer side of pass B, chunks downwards: for every own unknown, finish(dl, u, w, su, sw) with
 // su = sum_i cu[i] q_i, sw = sum_i cw[i] q_i and u = own slice of vector j
