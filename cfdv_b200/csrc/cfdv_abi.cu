@@ -547,7 +547,7 @@ int gmres_reference(cfdv_ctx* c, const cfdv_gmres_opts* o, cfdv_gmres_report* re
                 : reference_cycle_host(c, m, tol, h, &mm, &mag_r, rep);
     if (rc) return rc;
     tol = bnorm * 1.0E-9;
-    if (device && rep) rep->n_matvec += 1 + mm;
+    if (device && rep) rep->n_matvec += 1 + mm;  // the reference's count (cfdv_gpu.h)
     // the estimates of the cycle: c, s from the unrotated columns
     double est = mag_r;
     for (int j = 0; j < mm; j++) {

@@ -114,7 +114,10 @@ typedef struct {
   int gfinal_capacity;
   double* gfinal;      /* g(m) after each restart's rotation (MPI_GMRES.h:202-203) */
   int n_restarts;
-  int n_matvec;        /* EBE products issued */
+  int n_matvec;        /* EBE products.  CORRECT: issued.  REFERENCE: of the reference's iteration, one
+                        * a cycle for its residual and one a column; with m <= 62 the device leaves
+                        * out a zero start's residual and runs one product past a column at which
+                        * the estimate ends the cycle (solve_bytes of the profile counts what ran) */
   double true_rel_res; /* when requested */
 } cfdv_gmres_report;
 
