@@ -16,8 +16,21 @@ ADAPTIVE_CASES = ["lid8_adap", "plate20_adap", "ramp4_adap", "cyl4_adap"]  # eve
 GOLDEN = os.path.join(ROOT, "tests", "golden")
 
 
+def drop_stale_emulations(emu_dir, csrc_dir):
+    """Remove the CPU builds of kernel code that are older than any of the kernels' headers; the tests
+    that need one build it again.  Their own lists of headers need not follow what includes what."""
+    newest = max(os.path.getmtime(os.path.join(csrc_dir, f)) for f in os.listdir(csrc_dir)
+                 if f.endswith((".cuh", ".h")))
+    for f in os.listdir(emu_dir):
+        lib = os.path.join(emu_dir, f)
+        if f.startswith("lib") and f.endswith("_emu.so") and os.path.getmtime(lib) < newest:
+            os.remove(lib)
+
+
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200) and the built libcfdv_gpu.so")
+    if not hasattr(config, "workerinput"):  # once, before any parallel workers start
+        drop_stale_emulations(os.path.join(ROOT, "tests", "emu"), os.path.join(ROOT, "cfdv_b200", "csrc"))
 
 
 _cases = {}
