@@ -181,6 +181,14 @@ class ClockSampler:
                 "samples": len(sm)}
 
 
+def reference_missing():
+    """Why the reference build cannot be timed here, or None when it is there."""
+    from oracle import oracle as O
+    if os.path.exists(O.REF_BIN):
+        return None
+    return f"reference build missing: {os.path.relpath(O.REF_BIN, ROOT)} (made where the reference sources are)"
+
+
 def run_reference_cpu(case, steps, warmup):
     """Time the reference build on the host: (seconds per step list, sample description)."""
     from oracle import oracle as O
@@ -535,23 +543,35 @@ def bench_gpu(args, ws, rank, local):
         line["adjoint"] = measure_adjoint(args, ws, max_over_ranks)
     if rank == 0:
         if not args.no_cpu_baseline:
-            # the same sample as the reference arm's default: warm-up steps, then timed steps
-            k, w = CPU_SAMPLE.get(args.workload, (2, 1))
-            from cfdv_b200 import meshgen as mg
-            times = run_reference_cpu(WORKLOADS[args.workload]["make"](mg), k, w)
-            line["cpu_baseline"] = {"value": k / sum(times), "unit": "FDV steps/s", "cores": 1, "kind": "reference",
-                                    "cpu": cpu_model(),
-                                    "sample": f"{k} timed steps after {w} warm-up steps of the same case through "
-                                              f"oracle/_ref/cfdv_ref (reference sources, 1 core, the reference's "
-                                              f"GMRES({m}) with one restart: not equal residual)"}
+            line["cpu_baseline"] = cpu_baseline(args.workload)
         print(json.dumps(line))
     if ws > 1:
         import torch.distributed as dist
         dist.destroy_process_group()
 
 
+def cpu_baseline(workload):
+    """The reference build on one host core: the same sample as the reference arm's default (warm-up
+    steps, then timed steps)."""
+    missing = reference_missing()
+    if missing:
+        return {"unavailable": missing}
+    from cfdv_b200 import meshgen as mg
+    W = WORKLOADS[workload]
+    k, w = CPU_SAMPLE.get(workload, (2, 1))
+    times = run_reference_cpu(W["make"](mg), k, w)
+    return {"value": k / sum(times), "unit": "FDV steps/s", "cores": 1, "kind": "reference", "cpu": cpu_model(),
+            "sample": f"{k} timed steps after {w} warm-up steps of the same case through oracle/_ref/cfdv_ref "
+                      f"(reference sources, 1 core, the reference's GMRES({W['m']}) with one restart: not equal "
+                      f"residual)"}
+
+
 def bench_reference(args, ws, rank):
     if rank != 0:
+        return
+    missing = reference_missing()
+    if missing:
+        print(json.dumps({"impl": "reference", "unavailable": missing}))
         return
     from cfdv_b200 import meshgen as mg
     W = WORKLOADS[args.workload]
