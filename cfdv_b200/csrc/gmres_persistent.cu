@@ -1579,11 +1579,17 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_persistent_kernel(Persisten
 namespace {
 
 template <int KE, int NEQ, int NNOD, typename TR, bool RES>
-cudaError_t launch_cfg(const PersistentArgs& a, int blocks, size_t dyn_bytes, int node_cache, cudaStream_t st) {
+cudaError_t launch_cfg(const PersistentArgs& a, int blocks, int optin, size_t dyn_bytes, int node_cache,
+                       cudaStream_t st) {
   auto* k = gmres_persistent_kernel<KE, NEQ, NNOD, TR, RES, false>;
   if constexpr (sizeof(TR) == 8)
     if (a.ref_cycle) k = gmres_persistent_kernel<KE, NEQ, NNOD, TR, RES, true>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_bytes);
+  // the limit is the kernel's, not this launch's: always the most that the device allows, so that
+  // another thread's smaller launch cannot lower it between here and the launch
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaFuncGetAttributes(&fa, k);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, dyn_bytes);
@@ -1612,9 +1618,9 @@ cudaError_t launch_one(const PersistentArgs& a, cudaStream_t st) {
   // the node pass's offsets: an entry count and kMaxValence offsets per own node
   const size_t cache_bytes = (sizeof(int) * (size_t)pn * (kMaxValence + 1) + 7) / 8 * 8;
   if (cgs && a.max_valence <= kMaxValence && fa.sharedSizeBytes + res_bytes + cache_bytes <= (size_t)optin)
-    return launch_cfg<KE, NEQ, NNOD, TR, true>(a, blocks, res_bytes + cache_bytes, 1, st);
+    return launch_cfg<KE, NEQ, NNOD, TR, true>(a, blocks, optin, res_bytes + cache_bytes, 1, st);
   if (cgs && fa.sharedSizeBytes + res_bytes <= (size_t)optin)
-    return launch_cfg<KE, NEQ, NNOD, TR, true>(a, blocks, res_bytes, 0, st);
+    return launch_cfg<KE, NEQ, NNOD, TR, true>(a, blocks, optin, res_bytes, 0, st);
   e = cudaFuncGetAttributes(&fa, gmres_persistent_kernel<KE, NEQ, NNOD, TR, false, false>);
   if (e != cudaSuccess) return e;
   const bool dcgs = KE == 40 && cgs && a.orth != 0;  // the basis through the ring
@@ -1631,7 +1637,7 @@ cudaError_t launch_one(const PersistentArgs& a, cudaStream_t st) {
         ar.ring_stage_bytes = (int)(se * kElem64);
         ar.gs_offset = 0;
         ar.gs_bytes = dcgs ? ring_xbuf_offset(se * kElem64) : 0;
-        return launch_cfg<KE, NEQ, NNOD, TR, false>(ar, blocks, ring_bytes, 0, st);
+        return launch_cfg<KE, NEQ, NNOD, TR, false>(ar, blocks, optin, ring_bytes, 0, st);
       }
     }
   }
@@ -1645,7 +1651,7 @@ cudaError_t launch_one(const PersistentArgs& a, cudaStream_t st) {
     const size_t most = ((size_t)optin - fa.sharedSizeBytes - str_bytes) / slot;
     ad.gs_bytes = slot * (most < 4 ? most : 4);
   }
-  return launch_cfg<KE, NEQ, NNOD, TR, false>(ad, blocks, str_bytes + ad.gs_bytes, 0, st);
+  return launch_cfg<KE, NEQ, NNOD, TR, false>(ad, blocks, optin, str_bytes + ad.gs_bytes, 0, st);
 }
 
 cudaError_t launch_dim(int ndim, int fp32, const PersistentArgs& a, cudaStream_t st) {
