@@ -66,7 +66,7 @@ CFDV_HD CFDV_INLINE void jac_apply(const Dual* J, const Dual& f, const V* x, Dua
   }
 }
 
-// y += s2 a_I u1_I + s4 b_I u1_I and gam[i] += c_iI u1_I is formed row-wise below
+// y += s4 b_I u1_I (the a part is added for all directions at once, in jvp_point)
 template <int NDIM, int I>
 CFDV_HD CFDV_INLINE void jvp_beta(const GasT<Dual>& g, const GpStateT<Dual>& f, const Dual* s, const double (*u1)[5],
                                   Dual* y) {

@@ -19,8 +19,8 @@ namespace cfdv {
 // below leaves the normal numbers then, the residual of about 2^-53 x among them.  A zero's quotient is
 // the first product, its sign with it (Dirichlet rows are zeros: sent to the division they cost a mixed
 // solve 1%); anything else (infinite, NaN, tiny, huge) takes the division itself.  A numerator's range
-// is read off its exponent's word: mixed solves of 16,800 to 72,000 hexes take 0.9 to 1.7% less than
-// with a check of the divisor alone, FP64 ones as long within 0.3%.
+// is read off its exponent's word: two comparisons of the value cost FP64 solves of 16,800 to 72,000
+// hexes 0.4 to 0.9%.
 struct Divisor {
   double d, rd;
   bool fast;

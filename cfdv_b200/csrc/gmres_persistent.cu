@@ -4,7 +4,7 @@
 // host costs more than the arithmetic on the 2D cases (they fit in L2), and on the 3D
 // cases the host round trips still idle the GPU between passes.  This kernel keeps the
 // whole solve on the device: every restart recomputes r = b - A du with the FP64
-// matrices, then runs the Arnoldi cycle, applies the Givens rotations, tests
+// matrices (from a zero start a streamed basis takes r = b), then runs the Arnoldi cycle, applies the Givens rotations, tests
 // |g_{j+1}| < rtol ||b|| (the stopping rule of the textbook solver), back-substitutes the
 // small triangular system and adds P V y to du.  Products use the FP64 matrices, or the
 // FP32 matrices with FP32 accumulation for the mixed form (the restart residual stays
@@ -25,8 +25,9 @@
 // no block waits for another to publish those scalars.  Block 0 alone records H, the
 // residual estimates and the counters.
 //
-// Orthogonalisation: classical Gram-Schmidt applied twice (CGS2, the default) or modified
-// Gram-Schmidt (MGS), both with FP64 dots and norms.  CGS2 reduces the j+1 projections of
+// Orthogonalisation: classical Gram-Schmidt applied twice, the second pass delayed to the next step
+// (DCGS2, the default, at the Arnoldi loop below) or not (CGS2), or modified Gram-Schmidt (MGS), all
+// with FP64 dots and norms.  CGS2 reduces the j+1 projections of
 // a pass at once and repeats the pass once ("twice is enough": orthogonality to working
 // precision, as with MGS).  The norm of the new vector comes from the second pass's
 // partials, ||w2||^2 = ||w1||^2 - ||h2||^2 (w2 = w1 - V h2 with V orthonormal); when that
@@ -610,9 +611,9 @@ __device__ __forceinline__ void gs_pass_b(const GsRing& r, int j, const double* 
 // 2D (L2-resident, latency-bound): the block's warps form groups of G = lcm(Ke, 32) / 32
 // warps (one warp, two elements) that each take U = 3 waves of their elements at once from
 // the block's contiguous range (the block's whole share in one chunk), synchronising only
-// within the group.  3D (streamed from HBM): waves of kThreads / Ke elements interleaved over
-// the grid with a block barrier per wave; this kept more of the HBM bandwidth than
-// independent groups or bulk L2 prefetches of the next waves did.  x_e of a wave is gathered
+// within the group.  3D: waves of kThreads / Ke elements interleaved over the grid with a block
+// barrier per wave, for a resident basis (small meshes); a streamed one goes through elem_pass_ring
+// above, and comes here only with PersistentArgs::ring = 0.  x_e of a wave is gathered
 // into a shared tile; the gather offsets of the first chunk are kept from launch start
 // (`first`, shared memory).
 template <int KE>

@@ -1,8 +1,8 @@
 // Neighbour sets of the persistent GMRES solve's delayed-CGS2 step (gmres_persistent.cu), host
-// only.  Block b of the solve owns nodes [b pn, (b+1) pn), pn = ceil(n_nodes / nb), and in 2D
-// elements [b per, (b+1) per), per = ceil(E / nb).  Its element pass reads x at the nodes of its
+// only.  In 2D block b of the solve owns nodes [b pn, (b+1) pn), pn = ceil(n_nodes / nb), and elements
+// [b per, (b+1) per), per = ceil(E / nb).  Its element pass reads x at the nodes of its
 // elements and its node pass reads the products of the elements at its nodes, so before each
-// it waits for the blocks that write those.
+// it waits for the blocks that write those.  In 3D it waits for the whole grid.
 #pragma once
 
 #include <algorithm>
@@ -12,7 +12,8 @@ namespace cfdv {
 
 // CSR over the blocks: rows [0, nb] list the blocks owning nodes of a block's elements, rows
 // [nb + 1, 2 nb + 1] the blocks owning elements at a block's nodes (a block itself excluded).
-// False when the sets do not apply (3D, whose element waves interleave over the grid) or when
+// False when the sets do not apply (3D: a resident basis takes its elements in waves interleaved over
+// the grid, a streamed one in contiguous ranges, with an even number of nodes a block) or when
 // a set has more than 32 blocks (one polling lane each).
 inline bool persistent_neighbour_sets(int ndim, int n_nodes, int n_elements, const int* conn, const int* csr_ptr,
                                       const int* csr_idx, int blocks, std::vector<int>& ptr, std::vector<int>& idx) {
